@@ -30,9 +30,9 @@ _DEFAULT_REFERENCE_DIR = "/root/reference"
 
 def reference_dir():
     """The reference source tree ($OPENPFC_REFERENCE_DIR, else the default
-    mount point), or None when it is absent."""
+    mount point), or None when it is absent or empty."""
     d = os.environ.get("OPENPFC_REFERENCE_DIR") or _DEFAULT_REFERENCE_DIR
-    return d if os.path.isdir(d) else None
+    return d if os.path.isdir(os.path.join(d, "include")) else None
 
 
 def build(ref: bool = True) -> None:
