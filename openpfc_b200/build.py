@@ -21,10 +21,10 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libopenpfc_b200.so")
-SOURCES = ["kernels_f32.cu", "kernels_f64.cu", "ensemble_f32.cu", "ensemble_f64.cu", "opfc.cu", "noalloc.cu",
+SOURCES = ["kernels_f32.cu", "kernels_f64.cu", "ensemble_f32.cu", "ensemble_f64.cu", "plane_f32.cu", "plane_f64.cu", "opfc.cu", "noalloc.cu",
            "ensemble.cu", "io.cu", "wait_check.cu"]
 HEADERS = ["fft_core.cuh", "kernels.cuh", "launch.h", "col_tma.cuh", "x_tma.cuh", "x_sq.cuh", "twiddle.h",
-           "ensemble.cuh", "autotune.h", "io.h"]
+           "ensemble.cuh", "autotune.h", "io.h", "plane.cuh", "plane.h"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
@@ -70,7 +70,7 @@ def _compile(src: str, extra) -> str:
     return obj
 
 
-def build(force: bool = False, jobs: int = 3, extra=()) -> str:
+def build(force: bool = False, jobs: int = 8, extra=()) -> str:
     os.makedirs(BUILD, exist_ok=True)
     if force:
         for f in os.listdir(BUILD):
@@ -88,7 +88,7 @@ def build(force: bool = False, jobs: int = 3, extra=()) -> str:
 def main(argv=None) -> int:
     ap = argparse.ArgumentParser()
     ap.add_argument("--force", action="store_true")
-    ap.add_argument("--jobs", type=int, default=3)
+    ap.add_argument("--jobs", type=int, default=8)
     ap.add_argument("--verbose-ptxas", action="store_true")
     a = ap.parse_args(argv)
     extra = ["-Xptxas", "-v"] if a.verbose_ptxas else []

@@ -28,6 +28,7 @@
 #include "../../include/openpfc_b200.h"
 #include "fft_core.cuh"
 #include "launch.h"
+#include "plane.h"
 #include "twiddle.h"
 #include "autotune.h"
 #include "io.h"
@@ -134,6 +135,7 @@ struct opfc_handle {
   void *real_buf = nullptr;  // real-space staging (N0 N1 N2 reals)
   unsigned int *flag = nullptr;
   double *partials = nullptr;
+  double *mean_dev = nullptr;  // mean density, read by the plane kernel of the step
   int npartials = 1184;
   size_t allocated = 0;
 
@@ -158,8 +160,9 @@ struct opfc_handle {
   void *adj_c[2] = {nullptr, nullptr};
   void *adj_r[4] = {nullptr, nullptr, nullptr, nullptr};
 
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t graph_exec = nullptr;
+  cudaGraphExec_t graph_exec = nullptr, graph_many = nullptr;  // one step, kGraphSteps steps
+  cudaStream_t side = nullptr;  // Hermitian projection beside the next step's passes
+  cudaEvent_t ev[2] = {nullptr, nullptr};
 
   bool use_tma = true;  // TMA-fed column passes (OPFC_NO_TMA=1 disables)
   // OPFC_NVTX=1: steps run eagerly (no CUDA graph) with one NVTX range per
@@ -182,6 +185,11 @@ struct opfc_handle {
   //        the folded tables and 128-byte rows (z length 1024, PLAIN and
   //        FILTERED; else as 7)
   int var_y = 0, var_x = 0, var_z = 0;
+  // the y inverse, x and y forward passes in one kernel, a kz plane per CTA
+  // (plane.cuh; plane_default or the autotuner decides)
+  bool plane = false;
+  // the transform's own x and y passes as one plane kernel
+  bool plane_fft = false;
   int num_sms = 148;
   struct Tmap {
     const void *ptr;
@@ -487,6 +495,7 @@ int prepare_a(opfc_handle *h) {
 
 // Number of kernels one step launches (YI, X, YF, ZU, HERM).
 constexpr int kStepKernels = 5;
+constexpr int kStepXY = 100;  // enqueue_step_kernels: the kernels before the z update
 const char *const kStepKernelNames[kStepKernels] = {"y_inverse", "x_fused", "y_forward",
                                                      "z_update", "hermitian_fix"};
 // NVTX range of each step kernel, named after the profiling regions of the
@@ -521,9 +530,116 @@ int enqueue_step(opfc_handle *h, int only = -1) {
   return OPFC_OK;
 }
 
+PlaneArgs plane_args(opfc_handle *h) {
+  PlaneArgs a{};
+  a.tw_x = h->tw_x;
+  a.tw_y = h->tw_y;
+  a.M = h->M;
+  a.n1 = h->n1;
+  a.n2 = h->n2;
+  a.nyq_off = h->nyq_off;
+  a.flag = h->flag;
+  return a;
+}
+
+// The fused x pass of the step (arrays, model and coefficients).
+XLaunch x_fused(opfc_handle *h) {
+  const int model = h->desc.model;
+  XLaunch X = x_base(h);
+  X.mode = X_FUSED;
+  X.in0 = h->work_a;
+  X.out = h->work_a;
+  X.mean = h->use_pass_mean ? h->pass_mean : mean_density(h);
+  if (model == OPFC_MODEL_PLAIN) {
+    X.model = MK_PLAIN;
+  } else if (model == OPFC_MODEL_FILTERED || user_ops_model(model)) {
+    X.model = MK_FILTERED;
+    X.c[0] = h->desc.p2 / 2.0;
+    X.c[1] = h->desc.p3 / 3.0;
+    X.c[2] = h->desc.p4 / 4.0;
+  } else if (model == OPFC_MODEL_ALUMINUM) {
+    // Aluminum.hpp:285-307 with the temperature offset T_var = 0 (G_grid = 0):
+    // N = p3_bar u^2 + p4_bar u^3 + q3 v^2 + q4_bar v^3 - stabP u,
+    // q3 = q31_bar T_const / T0 + q30_bar
+    X.model = MK_TUNGSTEN;
+    X.in1 = h->work_b;
+    const opfc_aluminum_params &p = h->desc.aluminum;
+    X.c[0] = p.p3_bar;
+    X.c[1] = p.p4_bar;
+    X.c[2] = p.q31_bar * p.T_const / p.T0 + p.q30_bar;
+    X.c[3] = p.q4_bar;
+    X.c[4] = p.stabP;
+    if (h->al_grad) {
+      // moving temperature: position- and time-dependent terms, third field
+      // P*psi (Aluminum.hpp:270-307); direct-load x kernel
+      X.model = MK_ALUMINUM_G;
+      X.in2 = h->work_c;
+      X.time = h->time_dev;
+      const double l = h->n0 * h->desc.dx[0];
+      const double al[18] = {h->desc.origin[0], h->desc.dx[0], l, std::floor(p.m_xpos / l) * l,
+                             std::fmod(p.m_xpos, l), p.G_grid, p.x_initial, p.V_grid, p.T0, p.T_const,
+                             p.q21_bar, p.q30_bar, p.q31_bar, p.p3_bar, p.p4_bar, p.q4_bar, p.stabP, h->pf0};
+      for (int i = 0; i < 18; ++i) X.al[i] = al[i];
+    }
+  } else {
+    X.model = MK_TUNGSTEN;
+    X.in1 = h->work_b;
+    const opfc_tungsten_params &p = h->desc.tungsten;
+    const double tau = p.T / p.T0;
+    const double p3b = p.shift_u * (p.p3 + 3 * p.shift_s * p.p4);
+    const double p4b = std::pow(p.shift_u, 2) * p.p4;
+    const double q30b = p.shift_u * (p.q30 + 3.0 * p.shift_s * p.q40);
+    const double q31b = p.shift_u * p.q31;
+    const double q40b = std::pow(p.shift_u, 2) * p.q40;
+    X.c[0] = p3b;
+    X.c[1] = p4b;
+    X.c[2] = q31b * tau + q30b;
+    X.c[3] = q40b;
+    X.c[4] = p.stabP;
+  }
+  return X;
+}
+
+// Whether y inverse, x and y forward can run as one plane kernel, and whether
+// they do when neither the autotuner nor the environment chose.
+bool plane_ok(const opfc_handle *h) {
+  return plane_fits(h->M, h->n1, (int)h->rsz, x_fused(const_cast<opfc_handle *>(h)).model);
+}
+bool plane_default(const opfc_handle *h) { return h->use_tma && plane_ok(h); }
+
+// The transform's plane kernel: where it fits and no pass is forced.
+bool plane_fft_default(const opfc_handle *h) {
+  const char *pv = std::getenv("OPFC_PLANE");
+  return h->use_tma && plane_fits(h->M, h->n1, (int)h->rsz, MK_PLAIN) && !std::getenv("OPFC_Y_VARIANT") &&
+         !std::getenv("OPFC_X_VARIANT") && !(pv && std::atoi(pv) != 1);
+}
+
+int plane_pass(opfc_handle *h) {
+  const XLaunch X = x_fused(h);
+  PlaneArgs a = plane_args(h);
+  a.in[0] = X.in0;
+  a.in[1] = X.in1;
+  a.in[2] = X.in2;
+  a.out = X.out;
+  a.scale = X.scale;
+  a.mean_dev = h->mean_dev;
+  std::copy(X.c, X.c + 5, a.c);
+  std::copy(X.al, X.al + 18, a.al);
+  a.time = X.time;
+  LAUNCH_TRY(h, h->prec == OPFC_FP64 ? launch_plane<double>(X.model, a, h->stream)
+                                     : launch_plane<float>(X.model, a, h->stream));
+  return OPFC_OK;
+}
+
 int enqueue_step_kernels(opfc_handle *h, int only) {
   const int model = h->desc.model;
-  if (only < 0 || only == 0) {  // YI
+  const bool plane = h->plane && (only < 0 || only == kStepXY);
+  const bool xy = only < 0 || only == kStepXY;  // y inverse, x, y forward
+  if (plane) {  // YI, X and YF
+    const int rc = plane_pass(h);
+    if (rc) return rc;
+  }
+  if (!plane && (xy || only == 0)) {  // YI
     if (two_field(model)) {
       LAUNCH_TRY(h, col_plain(h, 1, +1, h->work_a, h->work_a, h->work_b, h->work_b));
       if (h->al_grad) LAUNCH_TRY(h, col_plain(h, 1, +1, h->work_c, h->work_c));
@@ -531,62 +647,8 @@ int enqueue_step_kernels(opfc_handle *h, int only) {
       LAUNCH_TRY(h, col_plain(h, 1, +1, h->work_a, h->work_a));
     }
   }
-  if (only < 0 || only == 1) {  // X
-    XLaunch X = x_base(h);
-    X.mode = X_FUSED;
-    X.in0 = h->work_a;
-    X.out = h->work_a;
-    X.mean = h->use_pass_mean ? h->pass_mean : mean_density(h);
-    if (model == OPFC_MODEL_PLAIN) {
-      X.model = MK_PLAIN;
-    } else if (model == OPFC_MODEL_FILTERED || user_ops_model(model)) {
-      X.model = MK_FILTERED;
-      X.c[0] = h->desc.p2 / 2.0;
-      X.c[1] = h->desc.p3 / 3.0;
-      X.c[2] = h->desc.p4 / 4.0;
-    } else if (model == OPFC_MODEL_ALUMINUM) {
-      // Aluminum.hpp:285-307 with the temperature offset T_var = 0 (G_grid = 0):
-      // N = p3_bar u^2 + p4_bar u^3 + q3 v^2 + q4_bar v^3 - stabP u,
-      // q3 = q31_bar T_const / T0 + q30_bar
-      X.model = MK_TUNGSTEN;
-      X.in1 = h->work_b;
-      const opfc_aluminum_params &p = h->desc.aluminum;
-      X.c[0] = p.p3_bar;
-      X.c[1] = p.p4_bar;
-      X.c[2] = p.q31_bar * p.T_const / p.T0 + p.q30_bar;
-      X.c[3] = p.q4_bar;
-      X.c[4] = p.stabP;
-      if (h->al_grad) {
-        // moving temperature: position- and time-dependent terms, third field
-        // P*psi (Aluminum.hpp:270-307); direct-load x kernel
-        X.model = MK_ALUMINUM_G;
-        X.in2 = h->work_c;
-        X.time = h->time_dev;
-        const double l = h->n0 * h->desc.dx[0];
-        const double al[18] = {h->desc.origin[0], h->desc.dx[0], l, std::floor(p.m_xpos / l) * l,
-                               std::fmod(p.m_xpos, l), p.G_grid, p.x_initial, p.V_grid, p.T0, p.T_const,
-                               p.q21_bar, p.q30_bar, p.q31_bar, p.p3_bar, p.p4_bar, p.q4_bar, p.stabP, h->pf0};
-        for (int i = 0; i < 18; ++i) X.al[i] = al[i];
-      }
-    } else {
-      X.model = MK_TUNGSTEN;
-      X.in1 = h->work_b;
-      const opfc_tungsten_params &p = h->desc.tungsten;
-      const double tau = p.T / p.T0;
-      const double p3b = p.shift_u * (p.p3 + 3 * p.shift_s * p.p4);
-      const double p4b = std::pow(p.shift_u, 2) * p.p4;
-      const double q30b = p.shift_u * (p.q30 + 3.0 * p.shift_s * p.q40);
-      const double q31b = p.shift_u * p.q31;
-      const double q40b = std::pow(p.shift_u, 2) * p.q40;
-      X.c[0] = p3b;
-      X.c[1] = p4b;
-      X.c[2] = q31b * tau + q30b;
-      X.c[3] = q40b;
-      X.c[4] = p.stabP;
-    }
-    LAUNCH_TRY(h, xpass(h, X));
-  }
-  if (only < 0 || only == 2)  // YF
+  if (!plane && (xy || only == 1)) LAUNCH_TRY(h, xpass(h, x_fused(h)));
+  if (!plane && (xy || only == 2))  // YF
     LAUNCH_TRY(h, col_plain(h, 1, -1, h->work_a, h->work_a));
   if (only < 0 || only == 3) {  // ZU
     ColLaunch Z{};
@@ -667,16 +729,56 @@ int enqueue_step_kernels(opfc_handle *h, int only) {
 }
 
 void release_graph(opfc_handle *h) {
-  if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
-  if (h->graph) cudaGraphDestroy(h->graph);
-  h->graph_exec = nullptr;
-  h->graph = nullptr;
+  for (cudaGraphExec_t *g : {&h->graph_exec, &h->graph_many}) {
+    if (*g) cudaGraphExecDestroy(*g);
+    *g = nullptr;
+  }
 }
 
-int build_graph(opfc_handle *h) {
-  release_graph(h);
+// second stream of enqueue_steps (made outside any capture)
+int ensure_side(opfc_handle *h) {
+  if (!h->side) CUDA_TRY(h, cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
+  for (auto &e : h->ev)
+    if (!e) CUDA_TRY(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  return OPFC_OK;
+}
+
+// n steps on h->stream.  The Hermitian projection of a step touches psi_hat
+// only, which the next step reads in its z update, so it runs on a second
+// stream beside the next step's y and x passes and is joined before the z
+// update (and at the end).  It stays in line where it also advances the device
+// time, which the x pass reads.
+int enqueue_steps(opfc_handle *h, int n) {
+  int rc;
+  if (h->al_grad) {
+    for (int s = 0; s < n; ++s)
+      if ((rc = enqueue_step_kernels(h, -1))) return rc;
+    return OPFC_OK;
+  }
+  cudaStream_t main = h->stream;
+  for (int s = 0; s < n; ++s) {
+    if ((rc = enqueue_step_kernels(h, kStepXY))) return rc;
+    if (s > 0) CUDA_TRY(h, cudaStreamWaitEvent(main, h->ev[1], 0));
+    if ((rc = enqueue_step_kernels(h, 3))) return rc;
+    CUDA_TRY(h, cudaEventRecord(h->ev[0], main));
+    CUDA_TRY(h, cudaStreamWaitEvent(h->side, h->ev[0], 0));
+    h->stream = h->side;
+    rc = enqueue_step_kernels(h, 4);
+    h->stream = main;
+    if (rc) return rc;
+    CUDA_TRY(h, cudaEventRecord(h->ev[1], h->side));
+  }
+  CUDA_TRY(h, cudaStreamWaitEvent(main, h->ev[1], 0));
+  return OPFC_OK;
+}
+
+// Steps of one graph: a small grid's step is a few short kernels, so the gap
+// between graph launches would be a good part of it.
+constexpr int kGraphSteps = 10;
+
+int build_graph(opfc_handle *h, int steps, cudaGraphExec_t *exec) {
   CUDA_TRY(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  int rc = enqueue_step(h);
+  int rc = enqueue_steps(h, steps);
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(h->stream, &g);
   if (rc) {
@@ -684,10 +786,10 @@ int build_graph(opfc_handle *h) {
     return rc;
   }
   if (e != cudaSuccess) return fail(h, OPFC_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
-  h->graph = g;
-  e = cudaGraphInstantiate(&h->graph_exec, g, 0);
+  e = cudaGraphInstantiate(exec, g, 0);
+  cudaGraphDestroy(g);
   if (e != cudaSuccess) {
-    release_graph(h);
+    *exec = nullptr;
     return fail(h, OPFC_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
   }
   return OPFC_OK;
@@ -822,31 +924,90 @@ int user_sum(opfc_handle *h, const void *src, int dtype, int where, double *out)
   return OPFC_OK;
 }
 
-// real_buf -> work_a (forward R2C, full spectrum in the split layout)
-int forward_real_buf(opfc_handle *h, void *dst) {
+// Whether `p` can stand in for real_buf or a spectrum buffer in the passes: a
+// device array of the compute precision on a complex value's boundary (the
+// kernels move real rows as (x[2p], x[2p+1]) pairs).
+bool direct_ok(const opfc_handle *h, const void *p, int dtype, int where) {
+  return where == OPFC_DEVICE && (dtype == OPFC_F64) == (h->prec == OPFC_FP64) &&
+         reinterpret_cast<uintptr_t>(p) % (2 * h->rsz) == 0;
+}
+
+// real rows -> dst: x R2C, y forward
+int xy_forward(opfc_handle *h, const void *rin, void *dst) {
+  if (h->plane_fft) {
+    PlaneArgs a = plane_args(h);
+    a.rin = rin;
+    a.out = dst;
+    LAUNCH_TRY(h, h->prec == OPFC_FP64 ? launch_plane_fft<double>(-1, a, h->stream)
+                                       : launch_plane_fft<float>(-1, a, h->stream));
+    return OPFC_OK;
+  }
   XLaunch X = x_base(h);
   X.mode = X_R2C;
-  X.rin = h->real_buf;
+  X.rin = rin;
   X.out = dst;
   LAUNCH_TRY(h, xpass(h, X));
   LAUNCH_TRY(h, col_plain(h, 1, -1, dst, dst));
+  return OPFC_OK;
+}
+
+// src (z inverse done; left undefined) -> real rows: y inverse, x C2R, scaled by 1/N, + mean
+int xy_backward(opfc_handle *h, void *src, void *rout, double mean) {
+  XLaunch X = x_base(h);
+  if (h->plane_fft) {
+    PlaneArgs a = plane_args(h);
+    a.in[0] = src;
+    a.rout = rout;
+    a.scale = X.scale;
+    a.mean = mean;
+    LAUNCH_TRY(h, h->prec == OPFC_FP64 ? launch_plane_fft<double>(+1, a, h->stream)
+                                       : launch_plane_fft<float>(+1, a, h->stream));
+    return OPFC_OK;
+  }
+  LAUNCH_TRY(h, col_plain(h, 1, +1, src, src));
+  X.mode = X_C2R;
+  X.in0 = src;
+  X.rout = rout;
+  X.mean = mean;
+  LAUNCH_TRY(h, xpass(h, X));
+  return OPFC_OK;
+}
+
+// z transform of a whole spectrum between the split and the reference layout
+int z_ref(opfc_handle *h, int dir, const void *in, void *out) {
+  ZRefArgs a{};
+  a.in = in;
+  a.out = out;
+  a.tw = h->tw_z;
+  a.M = h->M;
+  a.n1 = h->n1;
+  a.n2 = h->n2;
+  a.nyq_off = h->nyq_off;
+  LAUNCH_TRY(h, h->prec == OPFC_FP64 ? launch_z_ref<double>(dir, a, h->stream) : launch_z_ref<float>(dir, a, h->stream));
+  return OPFC_OK;
+}
+
+// real rows -> dst (forward R2C, full spectrum in the split layout)
+int forward_real(opfc_handle *h, const void *rin, void *dst) {
+  const int rc = xy_forward(h, rin, dst);
+  if (rc) return rc;
   LAUNCH_TRY(h, col_plain(h, 2, -1, dst, dst));
   return OPFC_OK;
 }
 
-// src (split layout spectrum, z and y not yet inverted) -> real_buf, scaled, + mean
+// src (spectrum with the z inverse done; destroyed) -> the caller's field, scaled, + mean
+int backward_to_user(opfc_handle *h, void *src, double mean, void *dst, int dtype, int where) {
+  if (direct_ok(h, dst, dtype, where)) return xy_backward(h, src, dst, mean);
+  int rc = ensure_real_buf(h);
+  if (rc || (rc = xy_backward(h, src, h->real_buf, mean))) return rc;
+  return real_out(h, dst, dtype, where);
+}
+
+// src (split layout spectrum, y not yet inverted, z as z_done says) -> real_buf, scaled, + mean
 int backward_to_real_buf(opfc_handle *h, void *src, double mean, bool z_done) {
   if (!z_done) LAUNCH_TRY(h, col_plain(h, 2, +1, src, src));
-  LAUNCH_TRY(h, col_plain(h, 1, +1, src, src));
-  int rc = ensure_real_buf(h);
-  if (rc) return rc;
-  XLaunch X = x_base(h);
-  X.mode = X_C2R;
-  X.in0 = src;
-  X.rout = h->real_buf;
-  X.mean = mean;
-  LAUNCH_TRY(h, xpass(h, X));
-  return OPFC_OK;
+  const int rc = ensure_real_buf(h);
+  return rc ? rc : xy_backward(h, src, h->real_buf, mean);
 }
 
 }  // namespace
@@ -1041,6 +1202,9 @@ int opfc_destroy(opfc_handle *h) {
                  h->time_dev, h->fold_ops, h->fold_chi};
   for (void *p : adj)
     if (p) cudaFree(p);
+  for (cudaEvent_t e : h->ev)
+    if (e) cudaEventDestroy(e);
+  if (h->side) cudaStreamDestroy(h->side);
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
   cudaSetDevice(dev_prev);
   delete h;
@@ -1113,12 +1277,15 @@ int opfc_create(const opfc_desc *d, opfc_handle **out) {
   if ((rc = upload_twiddles(hp, hp->n1, &hp->tw_y))) return cleanup(rc);
   if ((rc = upload_twiddles(hp, hp->n2, &hp->tw_z))) return cleanup(rc);
   if ((rc = dev_alloc(hp, (void **)&hp->flag, sizeof(unsigned int)))) return cleanup(rc);
-  if ((rc = dev_alloc(hp, (void **)&hp->partials, sizeof(double) * hp->npartials))) return cleanup(rc);
+  // (the mean density follows the partial sums)
+  if ((rc = dev_alloc(hp, (void **)&hp->partials, sizeof(double) * (hp->npartials + 1)))) return cleanup(rc);
+  hp->mean_dev = hp->partials + hp->npartials;
   if (cudaMemset(hp->flag, 0, sizeof(unsigned int)) != cudaSuccess) return cleanup(OPFC_ERR_CUDA);
   if (cudaMemset(hp->psi_hat, 0, cb) != cudaSuccess) return cleanup(OPFC_ERR_CUDA);
   if (cudaDeviceGetAttribute(&hp->num_sms, cudaDevAttrMultiProcessorCount, hp->device) != cudaSuccess)
     hp->num_sms = 148;
   hp->tmaps.reserve(64);
+  hp->plane_fft = plane_fft_default(hp);
   *out = h.release();
   return OPFC_OK;
 }
@@ -1366,6 +1533,11 @@ static int finish_initialize(opfc_handle *h) {
     h->var_z = h->var_z == 4 ? 2 : 0;
   if (z_folded(h->var_z) && !h->fold_ops) h->var_z = h->var_z == 7 ? 2 : 0;
   if (h->var_y < 0 || h->var_y >= kVarY) h->var_y = 0;
+  // a forced y or x variant keeps the separate passes
+  const char *pv = std::getenv("OPFC_PLANE");
+  h->plane = AutoTuner::instance().get_config(tune_key(h, "xy"), plane_default(h)) == 1 && plane_ok(h) &&
+             !std::getenv("OPFC_Y_VARIANT") && !std::getenv("OPFC_X_VARIANT");
+  if (pv) h->plane = std::atoi(pv) == 1 && plane_ok(h);
   h->initialized = true;
   h->a_valid = false;
   release_graph(h);
@@ -1378,7 +1550,8 @@ int opfc_set_psi(opfc_handle *h, const void *psi, size_t count, int dtype, int w
   if ((rc = check_dtype_where(h, dtype, where))) return rc;
   if ((rc = check_count(h, count, h->nr, "opfc_set_psi"))) return rc;
   CUDA_TRY(h, cudaSetDevice(h->device));
-  if ((rc = real_in(h, psi, dtype, where))) return rc;
+  const bool direct = direct_ok(h, psi, dtype, where);
+  if (!direct && (rc = real_in(h, psi, dtype, where))) return rc;
   // k = 0 mode in FP64 with compensated summation of the caller's values in
   // their own precision (before any rounding to the compute precision).  A
   // host field already in the compute precision arrives bit for bit in the
@@ -1390,13 +1563,15 @@ int opfc_set_psi(opfc_handle *h, const void *psi, size_t count, int dtype, int w
   else
     rc = user_sum(h, psi, dtype, where, &h->mass_sum);
   if (rc) return rc;
-  if ((rc = forward_real_buf(h, h->psi_hat))) return rc;
+  if ((rc = forward_real(h, direct ? psi : h->real_buf, h->psi_hat))) return rc;
   // the DC slot of the FP32/FP64 array stays zero; mass_sum carries it
   CUDA_TRY(h, cudaMemsetAsync(h->psi_hat, 0, 2 * h->rsz, h->stream));
+  const double mean = mean_density(h);
+  CUDA_TRY(h, cudaMemcpyAsync(h->mean_dev, &mean, sizeof mean, cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   h->have_state = true;
   h->a_valid = false;
-  release_graph(h);  // the captured step bakes in the mean density
+  if (!h->plane) release_graph(h);  // the separate x pass bakes in the mean density
   return OPFC_OK;
 }
 
@@ -1408,9 +1583,8 @@ int opfc_get_psi(opfc_handle *h, void *psi, size_t count, int dtype, int where) 
   if (!h->have_state) return fail(h, OPFC_ERR_STATE, "opfc_get_psi before opfc_set_psi");
   CUDA_TRY(h, cudaSetDevice(h->device));
   LAUNCH_TRY(h, col_plain(h, 2, +1, h->psi_hat, h->work_a));
-  if ((rc = backward_to_real_buf(h, h->work_a, mean_density(h), true))) return rc;
   h->a_valid = false;
-  return real_out(h, psi, dtype, where);
+  return backward_to_user(h, h->work_a, mean_density(h), psi, dtype, where);
 }
 
 int opfc_get_psi_mf(opfc_handle *h, void *psi, size_t count, int dtype, int where) {
@@ -1472,10 +1646,18 @@ int opfc_step(opfc_handle *h, int n_steps) {
     }
     return OPFC_OK;
   }
-  if (!h->graph_exec) {
-    if ((rc = build_graph(h))) return rc;
+  if ((rc = ensure_side(h))) return rc;
+  // Without the plane kernel the mean density is a launch argument of the x
+  // pass, so a graph is captured again for every new field; from 2^20 cells on
+  // the kernels are long enough to hide their launches and no graph is needed.
+  if (!h->plane && h->nr >= ((size_t)1 << 20)) return enqueue_steps(h, n_steps);
+  while (n_steps > 0) {
+    const bool many = n_steps >= kGraphSteps;
+    cudaGraphExec_t *g = many ? &h->graph_many : &h->graph_exec;
+    if (!*g && (rc = build_graph(h, many ? kGraphSteps : 1, g))) return rc;
+    CUDA_TRY(h, cudaGraphLaunch(*g, h->stream));
+    n_steps -= many ? kGraphSteps : 1;
   }
-  for (int s = 0; s < n_steps; ++s) CUDA_TRY(h, cudaGraphLaunch(h->graph_exec, h->stream));
   return OPFC_OK;
 }
 
@@ -1574,9 +1756,10 @@ int opfc_fft_forward(opfc_handle *h, const void *in_real, void *out_complex, int
   int rc;
   if ((rc = check_dtype_where(h, dtype, where))) return rc;
   CUDA_TRY(h, cudaSetDevice(h->device));
-  if ((rc = real_in(h, in_real, dtype, where))) return rc;
-  if ((rc = forward_real_buf(h, h->work_a))) return rc;
+  const bool direct = direct_ok(h, in_real, dtype, where);
+  if (!direct && (rc = real_in(h, in_real, dtype, where))) return rc;
   h->a_valid = false;
+  if ((rc = xy_forward(h, direct ? in_real : h->real_buf, h->work_a))) return rc;
   const size_t esz = dtype == OPFC_F64 ? 8 : 4;
   void *dst = out_complex, *tmp = nullptr;
   if (where == OPFC_HOST) {
@@ -1584,11 +1767,16 @@ int opfc_fft_forward(opfc_handle *h, const void *in_real, void *out_complex, int
     dst = tmp;
   }
   const int f64 = dtype == OPFC_F64;
-  if (h->prec == OPFC_FP64)
-    rc = launch_to_ref<double>(h->work_a, dst, f64, h->M, h->n1, h->n2, h->nyq_off, 0, 0.0, h->stream);
-  else
-    rc = launch_to_ref<float>(h->work_a, dst, f64, h->M, h->n1, h->n2, h->nyq_off, 0, 0.0, h->stream);
-  if (rc) return fail(h, OPFC_ERR_CUDA, "to_ref: %s", cudaGetErrorString((cudaError_t)rc));
+  if (direct_ok(h, dst, dtype, OPFC_DEVICE)) {
+    if ((rc = z_ref(h, -1, h->work_a, dst))) return rc;
+  } else {
+    LAUNCH_TRY(h, col_plain(h, 2, -1, h->work_a, h->work_a));
+    if (h->prec == OPFC_FP64)
+      rc = launch_to_ref<double>(h->work_a, dst, f64, h->M, h->n1, h->n2, h->nyq_off, 0, 0.0, h->stream);
+    else
+      rc = launch_to_ref<float>(h->work_a, dst, f64, h->M, h->n1, h->n2, h->nyq_off, 0, 0.0, h->stream);
+    if (rc) return fail(h, OPFC_ERR_CUDA, "to_ref: %s", cudaGetErrorString((cudaError_t)rc));
+  }
   if (tmp) {
     CUDA_TRY(h, cudaMemcpyAsync(out_complex, tmp, h->nc * 2 * esz, cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(h, cudaFreeAsync(tmp, h->stream));
@@ -1611,15 +1799,19 @@ int opfc_fft_backward(opfc_handle *h, const void *in_complex, void *out_real, in
     src = tmp;
   }
   const int f64 = dtype == OPFC_F64;
-  if (h->prec == OPFC_FP64)
-    rc = launch_from_ref<double>(src, f64, h->work_a, h->M, h->n1, h->n2, h->nyq_off, h->stream);
-  else
-    rc = launch_from_ref<float>(src, f64, h->work_a, h->M, h->n1, h->n2, h->nyq_off, h->stream);
-  if (rc) return fail(h, OPFC_ERR_CUDA, "from_ref: %s", cudaGetErrorString((cudaError_t)rc));
-  if (tmp) CUDA_TRY(h, cudaFreeAsync(tmp, h->stream));
   h->a_valid = false;
-  if ((rc = backward_to_real_buf(h, h->work_a, 0.0, false))) return rc;
-  return real_out(h, out_real, dtype, where);
+  if (direct_ok(h, src, dtype, OPFC_DEVICE)) {
+    if ((rc = z_ref(h, +1, src, h->work_a))) return rc;
+  } else {
+    if (h->prec == OPFC_FP64)
+      rc = launch_from_ref<double>(src, f64, h->work_a, h->M, h->n1, h->n2, h->nyq_off, h->stream);
+    else
+      rc = launch_from_ref<float>(src, f64, h->work_a, h->M, h->n1, h->n2, h->nyq_off, h->stream);
+    if (rc) return fail(h, OPFC_ERR_CUDA, "from_ref: %s", cudaGetErrorString((cudaError_t)rc));
+    LAUNCH_TRY(h, col_plain(h, 2, +1, h->work_a, h->work_a));
+  }
+  if (tmp) CUDA_TRY(h, cudaFreeAsync(tmp, h->stream));
+  return backward_to_user(h, h->work_a, 0.0, out_real, dtype, where);
 }
 
 int opfc_mass(opfc_handle *h, double *mean) {
@@ -1673,6 +1865,7 @@ int opfc_kernels_per_step(const opfc_handle *h) {
   const bool ring = h->var_z == 9 && h->n2 == 1024 && h->fold_ops && h->use_tma && !h->al_grad &&
                     (model == OPFC_MODEL_PLAIN || model == OPFC_MODEL_FILTERED) &&
                     h->M % (128 / (2 * (int)h->rsz)) == 0;
+  if (h->plane) return kStepKernels - 2 + (ring ? 1 : 0);
   return kStepKernels + (h->al_grad ? 1 : 0) + (ring ? 1 : 0);
 }
 
@@ -1686,6 +1879,18 @@ int opfc_autotune(opfc_handle *h, double *ms) {
   // each candidate runs its pass alone, in place on whatever the arrays hold
   h->var_y = T.tune(tune_key(h, "y"), kVarY, [&](int v) { h->var_y = v; return enqueue_step(h, 0); }, h->stream, &my);
   h->var_x = T.tune(tune_key(h, "x"), kVarX, [&](int v) { h->var_x = v; return enqueue_step(h, 1); }, h->stream, &mx);
+  // 0: those two passes as three launches, 1: the plane kernel
+  h->plane = false;
+  if (plane_ok(h))
+    h->plane = T.tune(
+                   tune_key(h, "xy"), 2,
+                   [&](int v) {
+                     if (v == 1) return plane_pass(h);
+                     int rc = 0;
+                     for (int k = 0; k < 3 && !rc; ++k) rc = enqueue_step(h, k);
+                     return rc;
+                   },
+                   h->stream) == 1;
   h->var_z = T.tune(
       tune_key(h, "z"), kVarZ,
       [&](int v) {
@@ -2088,28 +2293,12 @@ namespace {
 const int kEltBlocks = 148 * 8;
 
 // real `in` (device, compute precision) -> split-layout spectrum `out`
-int fwd_real(opfc_handle *h, const void *in, void *out) {
-  XLaunch X = x_base(h);
-  X.mode = X_R2C;
-  X.rin = in;
-  X.out = out;
-  LAUNCH_TRY(h, xpass(h, X));
-  LAUNCH_TRY(h, col_plain(h, 1, -1, out, out));
-  LAUNCH_TRY(h, col_plain(h, 2, -1, out, out));
-  return OPFC_OK;
-}
+int fwd_real(opfc_handle *h, const void *in, void *out) { return forward_real(h, in, out); }
 
 // split-layout spectrum `spec` (destroyed) -> real `out`, scaled by 1/N, + mean
 int bwd_real(opfc_handle *h, void *spec, void *out, double mean) {
   LAUNCH_TRY(h, col_plain(h, 2, +1, spec, spec));
-  LAUNCH_TRY(h, col_plain(h, 1, +1, spec, spec));
-  XLaunch X = x_base(h);
-  X.mode = X_C2R;
-  X.in0 = spec;
-  X.rout = out;
-  X.mean = mean;
-  LAUNCH_TRY(h, xpass(h, X));
-  return OPFC_OK;
+  return xy_backward(h, spec, out, mean);
 }
 
 // phi'(x) for phi(x) = (e^x - 1)/x, stable near 0

@@ -1,0 +1,7 @@
+// plane kernel, FP32 instantiation (see plane.cuh)
+#include "plane.cuh"
+namespace opfc {
+template int launch_plane<float>(int, const PlaneArgs &, cudaStream_t);
+template int launch_plane_fft<float>(int, const PlaneArgs &, cudaStream_t);
+template int launch_z_ref<float>(int, const ZRefArgs &, cudaStream_t);
+}

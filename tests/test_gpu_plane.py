@@ -1,0 +1,96 @@
+"""The plane kernel (y inverse, x and y forward of one kz plane in shared memory)
+against the oracle: every model, both precisions, plane sides of every plan
+(powers of two and mixed lengths, one line per turn up to several), and the
+transform's own plane and z kernels.  Tolerances as in the other parity tests:
+FP64 rounding over the steps, FP32 its own rounding level."""
+import math
+
+import numpy as np
+import pytest
+
+import openpfc_b200 as ob
+
+pytestmark = pytest.mark.gpu
+
+PI4 = [math.pi / 4] * 3
+TOL = {ob.FP64: 1e-11, ob.FP32: 1e-5}
+# (n0, n1, n2): smallest plane; mixed lengths on either side; turns of unequal
+# length (65 columns); 512-point lines; a plane near the shared-memory limit
+SHAPES = [(32, 16, 16), (48, 80, 16), (80, 24, 32), (192, 40, 16), (96, 96, 2), (128, 128, 16), (32, 512, 4),
+          (512, 48, 8), (1024, 16, 4), (160, 48, 1)]
+
+
+@pytest.fixture(autouse=True)
+def _plane(monkeypatch):
+    monkeypatch.setenv("OPENPFC_GPU_AUTOTUNE_MODE", "fallback_only")
+    monkeypatch.setenv("OPFC_PLANE", "1")
+
+
+def _rel(a, b):
+    return np.linalg.norm((a - b).ravel()) / np.linalg.norm(b.ravel())
+
+
+@pytest.mark.parametrize("prec", [ob.FP64, ob.FP32])
+@pytest.mark.parametrize("n", SHAPES)
+def test_plain(oracle, n, prec):
+    psi0 = ob.ic_noise(n, -0.285, 0.01, 3)
+    m = ob.PfcB200(n, PI4, r=-0.25, precision=prec)
+    m.initialize(0.5)
+    m.set_psi(psi0)
+    m.step(12)  # one graph of several steps, then single steps
+    m.sync()
+    assert _rel(m.get_psi(), oracle.run_plain(psi0, PI4, -0.25, 0.5, 12)) <= TOL[prec]
+    # the captured steps read the mean of the field set last
+    psi1 = ob.ic_noise(n, -0.2, 0.01, 4)
+    m.set_psi(psi1)
+    m.step(12)
+    m.sync()
+    assert _rel(m.get_psi(), oracle.run_plain(psi1, PI4, -0.25, 0.5, 12)) <= TOL[prec]
+
+
+@pytest.mark.parametrize("prec", [ob.FP64, ob.FP32])
+@pytest.mark.parametrize("n", [(32, 16, 16), (96, 40, 16), (64, 64, 16)])
+def test_filtered_and_tungsten(oracle, n, prec):
+    psi0 = ob.ic_noise(n, -0.10, 0.01, 5)
+    m = ob.FilteredB200(n, PI4, r=-0.3, alpha=0.5, p2=-0.1, p3=-0.5, p4=0.3, precision=prec)
+    m.initialize(0.5)
+    m.set_psi(psi0)
+    m.step(5)
+    m.sync()
+    ref = oracle.run_filtered(psi0, PI4, -0.3, 0.5, -0.1, -0.5, 0.3, 0.5, 5)
+    assert _rel(m.get_psi(), ref) <= TOL[prec]
+    dx = [1.1107207345395915] * 3
+    psi0 = ob.ic_noise(n, -0.40, 0.01, 6)
+    t = ob.TungstenB200(n, dx, precision=prec)
+    t.initialize(1.0)
+    t.set_psi(psi0)
+    t.step(5)
+    t.sync()
+    assert _rel(t.get_psi(), oracle.run_tungsten(psi0, dx, oracle.TungstenParams(), 1.0, 5)) <= TOL[prec]
+
+
+@pytest.mark.parametrize("n2", [1, 2, 16, 40, 48, 96, 256, 1024])
+@pytest.mark.parametrize("prec", [ob.FP64, ob.FP32])
+def test_transform_device_buffers(oracle, n2, prec):
+    """Device buffers of the compute precision go straight through the kernels;
+    an array off the complex boundary takes the copying path to the same values."""
+    import torch
+
+    n = (48, 16, n2)
+    dt = torch.float64 if prec == ob.FP64 else torch.float32
+    x = ob.ic_noise(n, 0.1, 1.0, 7)
+    f = ob.B200Fft(n, precision=prec)
+    ref = oracle.r2c(x)
+    pad = torch.empty(x.size + 1, dtype=dt, device="cuda")
+    for off in (0, 1):
+        dev = pad[off:off + x.size].view(n2, 16, 48)
+        dev.copy_(torch.from_numpy(x))
+        hat = torch.empty((n2, 16, 25, 2), dtype=dt, device="cuda")
+        torch.cuda.synchronize()
+        f.forward(dev, hat)
+        got = torch.view_as_complex(hat.double()).cpu().numpy()
+        assert np.abs(got - ref).max() <= (1e-12 if prec == ob.FP64 else 2e-6) * np.abs(ref).max()
+        back = torch.empty(x.size + 1, dtype=dt, device="cuda")[off:off + x.size].view(n2, 16, 48)
+        f.backward(hat, back)
+        torch.cuda.synchronize()
+        assert np.abs(back.double().cpu().numpy() - x).max() <= (1e-12 if prec == ob.FP64 else 2e-6) * np.abs(x).max()
