@@ -691,7 +691,9 @@ int enqueue_step_kernels(opfc_handle *h, int only) {
     // variant 9: 128-byte rows (the box-ring kernel's tensor maps)
     Z.wide = h->var_z == 9 && Z.fold_ops && !h->al_grad;
     const int W = Z.wide ? 128 / (2 * (int)h->rsz) : tma_col_width(Z.N, 2 * (int)h->rsz, COL_UPDATE);
-    if (h->use_tma && !h->al_grad && !z_direct(h->var_z) && Z.N > 1 && h->M % W == 0) {
+    // (at N = 2 a tile of a table is 64 bytes, and the next one would land off
+    // the 128-byte boundary that a TMA destination needs)
+    if (h->use_tma && !h->al_grad && !z_direct(h->var_z) && Z.N >= 4 && h->M % W == 0) {
       Z.tmap[0] = tmap_for(h, h->work_a, 2, W, false);
       Z.tmap[1] = tmap_for(h, h->psi_hat, 2, W, false);
       if (Z.computed) {
