@@ -16,6 +16,7 @@
 #include "../../include/openpfc_b200.h"
 #include "autotune.h"
 #include "ensemble.cuh"
+#include "host_pipe.h"
 #include "twiddle.h"
 
 using namespace opfc;
@@ -61,6 +62,7 @@ struct opfc_ensemble {
   int var_col = 0, var_x = 0, var_upd = 0;  // y passes, x pass, z update
   cudaGraphExec_t graph = nullptr;
   int graph_steps = 0;
+  HostPipe pipe;  // host arrays in and out
   std::string err;
   std::string key;
 };
@@ -399,14 +401,12 @@ int opfc_ensemble_set_psi(opfc_ensemble *e, int i, const double *psi, size_t cou
   const size_t nr = (size_t)in.n0 * in.n1 * in.n2;
   if (count != nr) return efail(e, OPFC_ERR_SIZE, "instance %d: expected %zu values", i, nr);
   ECUDA(e, cudaSetDevice(e->device));
-  in.mean = neumaier_sum(psi, nr) / (double)nr;
-  if (e->prec == OPFC_FP64) {
-    ECUDA(e, cudaMemcpyAsync(e->real_buf, psi, nr * 8, cudaMemcpyHostToDevice, e->stream));
-  } else {
-    std::vector<float> f(psi, psi + nr);
-    ECUDA(e, cudaMemcpyAsync(e->real_buf, f.data(), nr * 4, cudaMemcpyHostToDevice, e->stream));
-    ECUDA(e, cudaStreamSynchronize(e->stream));
-  }
+  std::vector<double> parts;
+  if (e->prec == OPFC_FP64)
+    ECUDA(e, e->pipe.in(e->device, psi, (double *)e->real_buf, nr, e->stream, &parts));
+  else
+    ECUDA(e, e->pipe.in(e->device, psi, (float *)e->real_buf, nr, e->stream, &parts));
+  in.mean = neumaier_sum(parts.data(), parts.size()) / (double)nr;
   XLaunch X = inst_x(e, in);
   X.mode = X_R2C;
   X.rin = e->real_buf;
@@ -442,13 +442,9 @@ int opfc_ensemble_get_psi(opfc_ensemble *e, int i, double *psi, size_t count) {
   if ((rc = x_run(e, X))) return rc;
   e->a_valid = false;
   if (e->prec == OPFC_FP64) {
-    ECUDA(e, cudaMemcpyAsync(psi, e->real_buf, nr * 8, cudaMemcpyDeviceToHost, e->stream));
-    ECUDA(e, cudaStreamSynchronize(e->stream));
+    ECUDA(e, e->pipe.out(e->device, (const double *)e->real_buf, psi, nr, e->stream));
   } else {
-    std::vector<float> f(nr);
-    ECUDA(e, cudaMemcpyAsync(f.data(), e->real_buf, nr * 4, cudaMemcpyDeviceToHost, e->stream));
-    ECUDA(e, cudaStreamSynchronize(e->stream));
-    for (size_t k = 0; k < nr; ++k) psi[k] = f[k];
+    ECUDA(e, e->pipe.out(e->device, (const float *)e->real_buf, psi, nr, e->stream));
   }
   return OPFC_OK;
 }

@@ -27,6 +27,7 @@
 
 #include "../../include/openpfc_b200.h"
 #include "fft_core.cuh"
+#include "host_pipe.h"
 #include "launch.h"
 #include "plane.h"
 #include "twiddle.h"
@@ -163,6 +164,7 @@ struct opfc_handle {
   cudaGraphExec_t graph_exec = nullptr, graph_many = nullptr;  // one step, kGraphSteps steps
   cudaStream_t side = nullptr;  // Hermitian projection beside the next step's passes
   cudaEvent_t ev[2] = {nullptr, nullptr};
+  HostPipe pipe;  // host arrays in and out
 
   bool use_tma = true;  // TMA-fed column passes (OPFC_NO_TMA=1 disables)
   // OPFC_NVTX=1: steps run eagerly (no CUDA graph) with one NVTX range per
@@ -814,67 +816,39 @@ int check_dtype_where(opfc_handle *h, int dtype, int where) {
   return OPFC_OK;
 }
 
-// copy a user real field (any dtype, host or device) into real_buf
-int real_in(opfc_handle *h, const void *src, int dtype, int where) {
+// copy a user real field (any dtype, host or device) into real_buf; with `parts`,
+// also append compensated partial sums of a host field's values
+int real_in(opfc_handle *h, const void *src, int dtype, int where, std::vector<double> *parts = nullptr) {
   int rc = ensure_real_buf(h);
   if (rc) return rc;
-  const bool same = (dtype == OPFC_F64) == (h->prec == OPFC_FP64);
+  const bool f64 = dtype == OPFC_F64, p64 = h->prec == OPFC_FP64;
   if (where == OPFC_HOST) {
-    if (same) {
-      CUDA_TRY(h, cudaMemcpyAsync(h->real_buf, src, h->nr * h->rsz, cudaMemcpyHostToDevice, h->stream));
-    } else if (h->prec == OPFC_FP64) {
-      std::vector<double> tmp(h->nr);
-      const float *f = (const float *)src;
-      for (size_t i = 0; i < h->nr; ++i) tmp[i] = f[i];
-      CUDA_TRY(h, cudaMemcpyAsync(h->real_buf, tmp.data(), h->nr * 8, cudaMemcpyHostToDevice, h->stream));
-      CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    } else {
-      std::vector<float> tmp(h->nr);
-      const double *d = (const double *)src;
-      for (size_t i = 0; i < h->nr; ++i) tmp[i] = (float)d[i];
-      CUDA_TRY(h, cudaMemcpyAsync(h->real_buf, tmp.data(), h->nr * 4, cudaMemcpyHostToDevice, h->stream));
-      CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    }
+    auto in = [&](auto *a, auto *b) { return h->pipe.in(h->device, a, b, h->nr, h->stream, parts); };
+    CUDA_TRY(h, f64 ? (p64 ? in((const double *)src, (double *)h->real_buf) : in((const double *)src, (float *)h->real_buf))
+                    : (p64 ? in((const float *)src, (double *)h->real_buf) : in((const float *)src, (float *)h->real_buf)));
+  } else if (f64 == p64) {
+    CUDA_TRY(h, cudaMemcpyAsync(h->real_buf, src, h->nr * h->rsz, cudaMemcpyDeviceToDevice, h->stream));
+  } else if (p64) {
+    LAUNCH_TRY(h, launch_cast_real<double>(src, 0, h->real_buf, 1, h->nr, h->stream));
   } else {
-    if (same) {
-      CUDA_TRY(h, cudaMemcpyAsync(h->real_buf, src, h->nr * h->rsz, cudaMemcpyDeviceToDevice, h->stream));
-    } else if (h->prec == OPFC_FP64) {
-      LAUNCH_TRY(h, launch_cast_real<double>(src, 0, h->real_buf, 1, h->nr, h->stream));
-    } else {
-      LAUNCH_TRY(h, launch_cast_real<float>(src, 1, h->real_buf, 0, h->nr, h->stream));
-    }
+    LAUNCH_TRY(h, launch_cast_real<float>(src, 1, h->real_buf, 0, h->nr, h->stream));
   }
   return OPFC_OK;
 }
 
 // copy real_buf out to a user buffer
 int real_out(opfc_handle *h, void *dst, int dtype, int where) {
-  const bool same = (dtype == OPFC_F64) == (h->prec == OPFC_FP64);
+  const bool f64 = dtype == OPFC_F64, p64 = h->prec == OPFC_FP64;
   if (where == OPFC_HOST) {
-    if (same) {
-      CUDA_TRY(h, cudaMemcpyAsync(dst, h->real_buf, h->nr * h->rsz, cudaMemcpyDeviceToHost, h->stream));
-      CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    } else if (h->prec == OPFC_FP64) {
-      std::vector<double> tmp(h->nr);
-      CUDA_TRY(h, cudaMemcpyAsync(tmp.data(), h->real_buf, h->nr * 8, cudaMemcpyDeviceToHost, h->stream));
-      CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-      float *f = (float *)dst;
-      for (size_t i = 0; i < h->nr; ++i) f[i] = (float)tmp[i];
-    } else {
-      std::vector<float> tmp(h->nr);
-      CUDA_TRY(h, cudaMemcpyAsync(tmp.data(), h->real_buf, h->nr * 4, cudaMemcpyDeviceToHost, h->stream));
-      CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-      double *d = (double *)dst;
-      for (size_t i = 0; i < h->nr; ++i) d[i] = tmp[i];
-    }
+    auto out = [&](auto *a, auto *b) { return h->pipe.out(h->device, a, b, h->nr, h->stream); };
+    CUDA_TRY(h, f64 ? (p64 ? out((const double *)h->real_buf, (double *)dst) : out((const float *)h->real_buf, (double *)dst))
+                    : (p64 ? out((const double *)h->real_buf, (float *)dst) : out((const float *)h->real_buf, (float *)dst)));
+  } else if (f64 == p64) {
+    CUDA_TRY(h, cudaMemcpyAsync(dst, h->real_buf, h->nr * h->rsz, cudaMemcpyDeviceToDevice, h->stream));
+  } else if (p64) {
+    LAUNCH_TRY(h, launch_cast_real<double>(h->real_buf, 1, dst, 0, h->nr, h->stream));
   } else {
-    if (same) {
-      CUDA_TRY(h, cudaMemcpyAsync(dst, h->real_buf, h->nr * h->rsz, cudaMemcpyDeviceToDevice, h->stream));
-    } else if (h->prec == OPFC_FP64) {
-      LAUNCH_TRY(h, launch_cast_real<double>(h->real_buf, 1, dst, 0, h->nr, h->stream));
-    } else {
-      LAUNCH_TRY(h, launch_cast_real<float>(h->real_buf, 0, dst, 1, h->nr, h->stream));
-    }
+    LAUNCH_TRY(h, launch_cast_real<float>(h->real_buf, 0, dst, 1, h->nr, h->stream));
   }
   return OPFC_OK;
 }
@@ -893,35 +867,16 @@ int device_sum(opfc_handle *h, int p, double *out) {
   return OPFC_OK;
 }
 
-// Compensated FP64 sum of a user field (host: threaded Neumaier chunks
-// combined with Neumaier; device: the FP64 reduction kernel in the field's dtype).
-int user_sum(opfc_handle *h, const void *src, int dtype, int where, double *out) {
-  if (where == OPFC_DEVICE) {
-    if (dtype == OPFC_F64)
-      LAUNCH_TRY(h, launch_sum_pow<double>(src, h->nr, 1, h->partials, h->npartials, h->stream));
-    else
-      LAUNCH_TRY(h, launch_sum_pow<float>(src, h->nr, 1, h->partials, h->npartials, h->stream));
-    std::vector<double> part(h->npartials);
-    CUDA_TRY(h, cudaMemcpyAsync(part.data(), h->partials, sizeof(double) * h->npartials,
-                                cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    *out = neumaier(part.data(), part.size());
-    return OPFC_OK;
-  }
-  const long nchunk = 64;
-  const size_t len = (h->nr + nchunk - 1) / nchunk;
-  std::vector<double> part(nchunk, 0.0);
-  parallel_for(nchunk, [&](long c) {
-    const size_t lo = (size_t)c * len, hi = std::min(h->nr, lo + len);
-    double s = 0, comp = 0;
-    for (size_t i = lo; i < hi; ++i) {
-      const double v = dtype == OPFC_F64 ? ((const double *)src)[i] : (double)((const float *)src)[i];
-      const double t = s + v;
-      comp += (std::fabs(s) >= std::fabs(v)) ? (s - t) + v : (v - t) + s;
-      s = t;
-    }
-    part[c] = s + comp;
-  });
+// Compensated FP64 sum of a device field, in its own precision.
+int user_sum(opfc_handle *h, const void *src, int dtype, double *out) {
+  if (dtype == OPFC_F64)
+    LAUNCH_TRY(h, launch_sum_pow<double>(src, h->nr, 1, h->partials, h->npartials, h->stream));
+  else
+    LAUNCH_TRY(h, launch_sum_pow<float>(src, h->nr, 1, h->partials, h->npartials, h->stream));
+  std::vector<double> part(h->npartials);
+  CUDA_TRY(h, cudaMemcpyAsync(part.data(), h->partials, sizeof(double) * h->npartials, cudaMemcpyDeviceToHost,
+                              h->stream));
+  CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   *out = neumaier(part.data(), part.size());
   return OPFC_OK;
 }
@@ -1553,18 +1508,19 @@ int opfc_set_psi(opfc_handle *h, const void *psi, size_t count, int dtype, int w
   if ((rc = check_count(h, count, h->nr, "opfc_set_psi"))) return rc;
   CUDA_TRY(h, cudaSetDevice(h->device));
   const bool direct = direct_ok(h, psi, dtype, where);
-  if (!direct && (rc = real_in(h, psi, dtype, where))) return rc;
   // k = 0 mode in FP64 with compensated summation of the caller's values in
   // their own precision (before any rounding to the compute precision).  A
   // host field already in the compute precision arrives bit for bit in the
-  // device buffer, so its sum runs there (one pass of the GPU) instead of on
-  // the host threads after the copy.
+  // device buffer, so its sum runs there; another one is summed by the host
+  // threads that convert it.
   const bool same_prec = (dtype == OPFC_F64) == (h->prec == OPFC_FP64);
-  if (where == OPFC_HOST && same_prec)
-    rc = user_sum(h, h->real_buf, dtype, OPFC_DEVICE, &h->mass_sum);
-  else
-    rc = user_sum(h, psi, dtype, where, &h->mass_sum);
-  if (rc) return rc;
+  const bool host_sum = where == OPFC_HOST && !same_prec;
+  std::vector<double> parts;
+  if (!direct && (rc = real_in(h, psi, dtype, where, host_sum ? &parts : nullptr))) return rc;
+  if (host_sum)
+    h->mass_sum = neumaier(parts.data(), parts.size());
+  else if ((rc = user_sum(h, where == OPFC_HOST ? h->real_buf : psi, dtype, &h->mass_sum)))
+    return rc;
   if ((rc = forward_real(h, direct ? psi : h->real_buf, h->psi_hat))) return rc;
   // the DC slot of the FP32/FP64 array stays zero; mass_sum carries it
   CUDA_TRY(h, cudaMemsetAsync(h->psi_hat, 0, 2 * h->rsz, h->stream));
