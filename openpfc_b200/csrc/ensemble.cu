@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
+#include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <string>
@@ -17,7 +18,15 @@
 #include "autotune.h"
 #include "ensemble.cuh"
 #include "host_pipe.h"
+#include "plane.h"
 #include "twiddle.h"
+
+namespace opfc {
+// plane kernel (ens_plane_f32.cu / ens_plane_f64.cu)
+template <typename Real> int ens_launch_plane(int planes, size_t smem, const EnsArgs &a, cudaStream_t s);
+extern template int ens_launch_plane<float>(int, size_t, const EnsArgs &, cudaStream_t);
+extern template int ens_launch_plane<double>(int, size_t, const EnsArgs &, cudaStream_t);
+}  // namespace opfc
 
 using namespace opfc;
 
@@ -58,6 +67,14 @@ struct opfc_ensemble {
   // transforms; mixing them thrashed the instruction cache) and the longest
   // tiles start first
   int *d_order[3] = {nullptr, nullptr, nullptr};
+  // plane kernel (y inverse, x and y forward in one launch): planes per member,
+  // prefix sums and order (largest plane first), the largest plane's shared memory
+  bool plane = true;
+  int planes = 0;
+  size_t plane_smem = 0;
+  int *d_prefix_plane = nullptr, *d_order_plane = nullptr;
+  cudaStream_t side = nullptr;  // Hermitian projection beside the next step's planes
+  cudaEvent_t ev[2] = {nullptr, nullptr};
   unsigned *flag = nullptr;
   int var_col = 0, var_x = 0, var_upd = 0;  // y passes, x pass, z update
   cudaGraphExec_t graph = nullptr;
@@ -132,12 +149,35 @@ int launch_stage(opfc_ensemble *e, int stage, int variant) {
                               : ens_launch_stage<float>(stage, W, G, e->num_sms, tiles, e->count, a, e->stream);
 }
 
-int enqueue_step(opfc_ensemble *e) {
-  const int v[5] = {e->var_col, e->var_x, e->var_col, e->var_upd, 0};
-  for (int s = 0; s < 5; ++s) {
-    const int rc = launch_stage(e, s, v[s]);
-    if (rc) return efail(e, OPFC_ERR_CUDA, "ensemble stage %d: %s", s, cudaGetErrorString((cudaError_t)rc));
+int launch_planes(opfc_ensemble *e) {
+  const EnsArgs a = args(e, e->d_prefix_plane, e->d_order_plane);
+  return e->prec == OPFC_FP64 ? ens_launch_plane<double>(e->planes, e->plane_smem, a, e->stream)
+                              : ens_launch_plane<float>(e->planes, e->plane_smem, a, e->stream);
+}
+
+// n steps; each step's Hermitian projection (psi_hat only, read next in the z
+// update) runs beside the next step's y and x passes
+int enqueue_steps(opfc_ensemble *e, int n) {
+  const cudaStream_t main = e->stream;
+  for (int i = 0; i < n; ++i) {
+    int rc = 0;
+    if (e->plane) {
+      rc = launch_planes(e);
+    } else {
+      const int v[3] = {e->var_col, e->var_x, e->var_col};
+      for (int s = 0; s < 3 && !rc; ++s) rc = launch_stage(e, s, v[s]);
+    }
+    if (i > 0) ECUDA(e, cudaStreamWaitEvent(main, e->ev[1], 0));
+    if (!rc) rc = launch_stage(e, 3, e->var_upd);
+    ECUDA(e, cudaEventRecord(e->ev[0], main));
+    ECUDA(e, cudaStreamWaitEvent(e->side, e->ev[0], 0));
+    e->stream = e->side;
+    if (!rc) rc = launch_stage(e, 4, 0);
+    e->stream = main;
+    ECUDA(e, cudaEventRecord(e->ev[1], e->side));
+    if (rc) return efail(e, OPFC_ERR_CUDA, "ensemble step: %s", cudaGetErrorString((cudaError_t)rc));
   }
+  ECUDA(e, cudaStreamWaitEvent(main, e->ev[1], 0));
   return OPFC_OK;
 }
 
@@ -245,9 +285,13 @@ int opfc_ensemble_destroy(opfc_ensemble *e) {
   drop_graph(e);
   void *bufs[] = {e->psi_hat, e->work, e->tw, e->real_buf, e->d_inst, e->flag,
                   e->d_prefix[0], e->d_prefix[1], e->d_prefix[2], e->d_prefix8[0], e->d_prefix8[1],
-                  e->d_prefix8[2], e->d_order[0], e->d_order[1], e->d_order[2]};
+                  e->d_prefix8[2], e->d_order[0], e->d_order[1], e->d_order[2], e->d_prefix_plane,
+                  e->d_order_plane};
   for (void *p : bufs)
     if (p) cudaFree(p);
+  for (cudaEvent_t v : e->ev)
+    if (v) cudaEventDestroy(v);
+  if (e->side) cudaStreamDestroy(e->side);
   if (e->own_stream && e->stream) cudaStreamDestroy(e->stream);
   delete e;
   return OPFC_OK;
@@ -362,6 +406,29 @@ int opfc_ensemble_create(int count, const opfc_desc *descs, opfc_ensemble **out)
         return bail(OPFC_ERR_CUDA);
     }
   }
+  {
+    std::vector<int> po(count), pre(count + 1, 0);
+    for (int i = 0; i < count; ++i) po[i] = i;
+    auto modes = [&](int i) { return (e->inst[i].M + 1) * e->inst[i].n1; };
+    std::stable_sort(po.begin(), po.end(), [&](int x, int y) { return modes(x) > modes(y); });
+    for (int k = 0; k < count; ++k) {
+      const EnsInst &in = e->inst[po[k]];
+      pre[k + 1] = pre[k] + in.n2;
+      ep->plane_smem = std::max(ep->plane_smem, plane_smem(in.M, in.n1, (int)e->rsz, MK_PLAIN));
+    }
+    ep->planes = pre[count];
+    if ((rc = ealloc(ep, (void **)&ep->d_order_plane, sizeof(int) * count)) ||
+        (rc = ealloc(ep, (void **)&ep->d_prefix_plane, sizeof(int) * (count + 1))))
+      return bail(rc);
+    if (cudaMemcpy(ep->d_order_plane, po.data(), sizeof(int) * count, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(ep->d_prefix_plane, pre.data(), sizeof(int) * (count + 1), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&ep->side, cudaStreamNonBlocking) != cudaSuccess)
+      return bail(OPFC_ERR_CUDA);
+    for (cudaEvent_t &v : ep->ev)
+      if (cudaEventCreateWithFlags(&v, cudaEventDisableTiming) != cudaSuccess) return bail(OPFC_ERR_CUDA);
+    const char *pv = std::getenv("OPFC_PLANE");
+    ep->plane = !(pv && pv[0] == '0') && AutoTuner::instance().get_config(e->key + "/xy", 1) == 1;
+  }
   if (cudaMemset(ep->flag, 0, sizeof(unsigned)) != cudaSuccess || cudaMemset(ep->psi_hat, 0, cb) != cudaSuccess ||
       cudaMemset(ep->work, 0, cb) != cudaSuccess)
     return bail(OPFC_ERR_CUDA);
@@ -462,7 +529,7 @@ int opfc_ensemble_step(opfc_ensemble *e, int n_steps) {
     drop_graph(e);
     // the whole n-step loop is one graph: 5 kernels per step
     ECUDA(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-    for (int s = 0; s < n_steps && !rc; ++s) rc = enqueue_step(e);
+    rc = enqueue_steps(e, n_steps);
     cudaGraph_t g = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(e->stream, &g);
     if (rc) {
@@ -502,6 +569,16 @@ int opfc_ensemble_autotune(opfc_ensemble *e, double *ms_col, double *ms_x, doubl
                                           [&](int v) { return launch_stage(e, 2, v); }, e->stream, &mc);
   e->var_x = AutoTuner::instance().tune(e->key + "/x", kVariants, [&](int v) { return launch_stage(e, 1, v); },
                                         e->stream, &mx);
+  // 0: the y, x and y passes, 1: the plane kernel
+  e->plane = AutoTuner::instance().tune(
+                 e->key + "/xy", 2,
+                 [&](int v) {
+                   if (v == 1) return launch_planes(e);
+                   int r = launch_stage(e, 0, e->var_col);
+                   if (!r) r = launch_stage(e, 1, e->var_x);
+                   return r ? r : launch_stage(e, 2, e->var_col);
+                 },
+                 e->stream) == 1;
   e->var_upd = AutoTuner::instance().tune(e->key + "/upd", kVariants,
                                           [&](int v) { return launch_stage(e, 3, v); }, e->stream, &mu);
   ECUDA(e, cudaStreamSynchronize(e->stream));

@@ -17,7 +17,7 @@ TOL = {ob.FP64: 1e-11, ob.FP32: 1e-5}
 # (n0, n1, n2): smallest plane; mixed lengths on either side; turns of unequal
 # length (65 columns); 512-point lines; a plane near the shared-memory limit
 SHAPES = [(32, 16, 16), (48, 80, 16), (80, 24, 32), (192, 40, 16), (96, 96, 2), (128, 128, 16), (32, 512, 4),
-          (512, 48, 8), (1024, 16, 4), (160, 48, 1)]
+          (512, 48, 8), (1024, 16, 4), (160, 48, 1), (64, 16, 40)]
 
 
 @pytest.fixture(autouse=True)
@@ -66,7 +66,7 @@ def test_filtered_and_tungsten(oracle, n, prec):
     t.set_psi(psi0)
     t.step(5)
     t.sync()
-    assert _rel(t.get_psi(), oracle.run_tungsten(psi0, dx, oracle.TungstenParams(), 1.0, 5)) <= TOL[prec]
+    assert _rel(t.get_psi(), oracle.run_tungsten(psi0, dx, oracle.TungstenParams.defaults(), 1.0, 5)) <= TOL[prec]
 
 
 @pytest.mark.parametrize("n2", [1, 2, 16, 40, 48, 96, 256, 1024])
@@ -94,3 +94,18 @@ def test_transform_device_buffers(oracle, n2, prec):
         f.backward(hat, back)
         torch.cuda.synchronize()
         assert np.abs(back.double().cpu().numpy() - x).max() <= (1e-12 if prec == ob.FP64 else 2e-6) * np.abs(x).max()
+
+
+@pytest.mark.parametrize("prec", [ob.FP64, ob.FP32])
+def test_ensemble(oracle, prec):
+    sides = [(32, 16, 48), (48, 96, 16), (80, 48, 32), (128, 128, 16), (96, 80, 16), (64, 64, 64)]
+    ms = [dict(n=s, dx=PI4, r=-0.2 - 0.02 * i) for i, s in enumerate(sides)]
+    e = ob.Ensemble(ms, precision=prec)
+    e.initialize(0.5)
+    psi = [ob.ic_noise(s, -0.285 + 0.01 * i, 0.01, 10 + i) for i, s in enumerate(sides)]
+    for i, p in enumerate(psi):
+        e.set_psi(i, p)
+    e.step(10)
+    e.sync()
+    for i, p in enumerate(psi):
+        assert _rel(e.get_psi(i), oracle.run_plain(p, PI4, ms[i]["r"], 0.5, 10)) <= TOL[prec]
