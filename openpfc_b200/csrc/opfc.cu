@@ -158,6 +158,11 @@ struct opfc_handle {
   // FP64-built per-mode tables folded by the evenness of k^2 in ky and kz
   void *fold_ops = nullptr, *fold_chi = nullptr;
   long long fold_nyq = 0;
+  // plane-kernel adjoint of the plain model: each step's F_z^-1[psi_hat] and
+  // F_xy[N] of the recomputed segment, and the z update's arrays meanwhile
+  std::vector<void *> seg_a, seg_n;
+  const void *z_in = nullptr;
+  void *z_out = nullptr;
   void *adj_c[2] = {nullptr, nullptr};
   void *adj_r[4] = {nullptr, nullptr, nullptr, nullptr};
 
@@ -616,8 +621,11 @@ bool plane_fft_default(const opfc_handle *h) {
          !std::getenv("OPFC_X_VARIANT") && !(pv && std::atoi(pv) != 1);
 }
 
-int plane_pass(opfc_handle *h) {
-  const XLaunch X = x_fused(h);
+// the step's plane kernel, work_a in place unless told otherwise
+int plane_pass(opfc_handle *h, const void *in = nullptr, void *out = nullptr) {
+  XLaunch X = x_fused(h);
+  if (in) X.in0 = in;
+  if (out) X.out = out;
   PlaneArgs a = plane_args(h);
   a.in[0] = X.in0;
   a.in[1] = X.in1;
@@ -664,8 +672,9 @@ int enqueue_step_kernels(opfc_handle *h, int only) {
     }
     Z.inverse_after = 1;
     Z.nsets = 1;
-    Z.in[0] = h->work_a;
-    Z.out[0] = h->work_a;
+    const void *zin = h->z_in ? h->z_in : h->work_a;
+    Z.in[0] = zin;
+    Z.out[0] = h->z_out ? h->z_out : h->work_a;
     Z.in[1] = h->work_b;
     Z.out[1] = h->work_b;
     Z.tw = h->tw_z;
@@ -696,7 +705,7 @@ int enqueue_step_kernels(opfc_handle *h, int only) {
     // (at N = 2 a tile of a table is 64 bytes, and the next one would land off
     // the 128-byte boundary that a TMA destination needs)
     if (h->use_tma && !h->al_grad && !z_direct(h->var_z) && Z.N >= 4 && h->M % W == 0) {
-      Z.tmap[0] = tmap_for(h, h->work_a, 2, W, false);
+      Z.tmap[0] = tmap_for(h, zin, 2, W, false);
       Z.tmap[1] = tmap_for(h, h->psi_hat, 2, W, false);
       if (Z.computed) {
         if (!Z.tmap[1]) Z.tmap[0] = nullptr;
@@ -775,6 +784,10 @@ int enqueue_steps(opfc_handle *h, int n) {
   CUDA_TRY(h, cudaStreamWaitEvent(main, h->ev[1], 0));
   return OPFC_OK;
 }
+
+// Whether the captured step outlives the field: these x passes read the mean
+// density from device memory; the others take it as a launch argument.
+bool keeps_graph(const opfc_handle *h) { return h->plane; }
 
 // Steps of one graph: a small grid's step is a few short kernels, so the gap
 // between graph launches would be a good part of it.
@@ -1152,8 +1165,9 @@ int opfc_destroy(opfc_handle *h) {
     if (p) cudaFree(p);
   for (void *p : h->ckpt)
     if (p) cudaFree(p);
-  for (void *p : h->seg)
-    if (p) cudaFree(p);
+  for (auto *v : {&h->seg, &h->seg_a, &h->seg_n})
+    for (void *p : *v)
+      if (p) cudaFree(p);
   void *adj[] = {h->tab_ar,   h->tab_br,   h->adj_c[0], h->adj_c[1], h->adj_r[0], h->adj_r[1],
                  h->adj_r[2], h->adj_r[3], h->rad_ops,  h->rad_chi,  h->tab_p,    h->work_c,
                  h->time_dev, h->fold_ops, h->fold_chi};
@@ -1529,7 +1543,7 @@ int opfc_set_psi(opfc_handle *h, const void *psi, size_t count, int dtype, int w
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   h->have_state = true;
   h->a_valid = false;
-  if (!h->plane) release_graph(h);  // the separate x pass bakes in the mean density
+  if (!keeps_graph(h)) release_graph(h);
   return OPFC_OK;
 }
 
@@ -1605,12 +1619,10 @@ int opfc_step(opfc_handle *h, int n_steps) {
     return OPFC_OK;
   }
   if ((rc = ensure_side(h))) return rc;
-  // Without the plane kernel the mean density is a launch argument of the x
-  // pass, so a graph is captured again for every new field; from 2^20 cells on
-  // the kernels are long enough to hide their launches and no graph is needed.
-  if (!h->plane && h->nr >= ((size_t)1 << 20)) return enqueue_steps(h, n_steps);
+  // From 2^21 cells on the separate passes are long enough to hide their launches.
+  if (!keeps_graph(h) && h->nr >= ((size_t)1 << 21)) return enqueue_steps(h, n_steps);
   while (n_steps > 0) {
-    const bool many = n_steps >= kGraphSteps;
+    const bool many = keeps_graph(h) && n_steps >= kGraphSteps;
     cudaGraphExec_t *g = many ? &h->graph_many : &h->graph_exec;
     if (!*g && (rc = build_graph(h, many ? kGraphSteps : 1, g))) return rc;
     CUDA_TRY(h, cudaGraphLaunch(*g, h->stream));
@@ -2210,6 +2222,28 @@ __global__ void adj_add_kernel(Real *lam, const Real *x, size_t n) {
 // U = opL lam_hat (in place over lam_hat), V = opN lam_hat (over n_hat, after
 // it is read), and (tar != nullptr) FP64 sums of w_kx Re(conj(lam_hat)(dA psi_hat
 // + dB n_hat)) added to this block's running partial.
+// r-derivatives of the tables, built where they are used (one FP64 exp and expm1
+// per mode; the host took milliseconds at 128^3 and copied them over):
+// d opL/dr = -k^2 dt e^{L dt}, d opN/dr = dt^2 k^4 phi'(L dt), phi(x) = (e^x - 1)/x
+template <typename Real>
+__global__ void adj_tables_kernel(Real *ar, Real *br, int M, int n1, int n2, long long nyq_off, double f0, double f1,
+                                  double f2, double r, double dt) {
+  const long long nc = nyq_off + (long long)n1 * n2;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nc;
+       i += (long long)gridDim.x * blockDim.x) {
+    const long long row = i < nyq_off ? i / M : i - nyq_off;
+    const int kx = i < nyq_off ? (int)(i - row * M) : M, ky = (int)(row % n1), kz = (int)(row / n1);
+    const double a = kx * f0, b = (ky <= n1 / 2 ? ky : ky - n1) * f1, c = (kz <= n2 / 2 ? kz : kz - n2) * f2;
+    const double k2 = a * a + b * b + c * c;
+    const double x = -k2 * (r + (1.0 - k2) * (1.0 - k2)) * dt;
+    // phi', stable near 0
+    const double e = exp(x);
+    const double dphi = fabs(x) < 1e-4 ? 0.5 + x / 3.0 + x * x / 8.0 + x * x * x / 30.0 : (x * e - expm1(x)) / (x * x);
+    ar[i] = (Real)(-k2 * dt * e);
+    br[i] = (Real)(dt * dt * k2 * k2 * dphi);
+  }
+}
+
 template <typename Real>
 __global__ void adj_modes_kernel(typename opfc::Cx<Real>::T *lam_hat, const typename opfc::Cx<Real>::T *psi_hat,
                                  typename opfc::Cx<Real>::T *n_hat, const Real *ta, const Real *tb,
@@ -2259,12 +2293,6 @@ int bwd_real(opfc_handle *h, void *spec, void *out, double mean) {
   return xy_backward(h, spec, out, mean);
 }
 
-// phi'(x) for phi(x) = (e^x - 1)/x, stable near 0
-double dphi(double x) {
-  if (std::fabs(x) < 1e-4) return 0.5 + x / 3.0 + x * x / 8.0 + x * x * x / 30.0;
-  return (x * std::exp(x) - std::expm1(x)) / (x * x);
-}
-
 // models whose operators depend on r (L = -k^2 (r + (1 - k^2)^2))
 bool has_r(const opfc_handle *h) {
   return h->desc.model == OPFC_MODEL_PLAIN || h->desc.model == OPFC_MODEL_FILTERED;
@@ -2302,38 +2330,20 @@ int adj_kind(const opfc_handle *h, double c[5]) {
 
 int adjoint_tables(opfc_handle *h) {
   if (!has_r(h)) return OPFC_OK;  // no r-derivative tables
-  const int n0 = h->n0, n1 = h->n1, n2 = h->n2, H = h->M + 1;
-  const double f0 = 2.0 * kPi / (h->desc.dx[0] * n0);
-  const double f1 = 2.0 * kPi / (h->desc.dx[1] * n1);
-  const double f2 = 2.0 * kPi / (h->desc.dx[2] * n2);
-  const double r = h->desc.r, dt = h->dt;
-  std::vector<double> ar(h->nc), br(h->nc);
-  auto kc = [](int i, int n, double f) { return (i <= n / 2) ? i * f : (i - n) * f; };
-  parallel_for((long)n2 * n1, [&](long row) {
-    const int ky = (int)(row % n1), kz = (int)(row / n1);
-    for (int kx = 0; kx < H; ++kx) {
-      const double a = kc(kx, n0, f0), b = kc(ky, n1, f1), c = kc(kz, n2, f2);
-      const double k2 = a * a + b * b + c * c;
-      const double L = -k2 * (r + (1.0 - k2) * (1.0 - k2));
-      const size_t o = split_index(h, kx, ky, kz);
-      ar[o] = -k2 * dt * std::exp(L * dt);
-      br[o] = dt * dt * k2 * k2 * dphi(L * dt);
-    }
-  });
-  for (int t = 0; t < 2; ++t) {
-    void **dst = t == 0 ? &h->tab_ar : &h->tab_br;
-    std::vector<double> &src = t == 0 ? ar : br;
+  for (void **dst : {&h->tab_ar, &h->tab_br})
     if (!*dst) {
-      int rc = dev_alloc(h, dst, h->nc * h->rsz);
+      const int rc = dev_alloc(h, dst, h->nc * h->rsz);
       if (rc) return rc;
     }
-    if (h->prec == OPFC_FP64) {
-      CUDA_TRY(h, cudaMemcpy(*dst, src.data(), h->nc * 8, cudaMemcpyHostToDevice));
-    } else {
-      std::vector<float> f(src.begin(), src.end());
-      CUDA_TRY(h, cudaMemcpy(*dst, f.data(), h->nc * 4, cudaMemcpyHostToDevice));
-    }
-  }
+  const double f0 = 2.0 * kPi / (h->desc.dx[0] * h->n0), f1 = 2.0 * kPi / (h->desc.dx[1] * h->n1),
+               f2 = 2.0 * kPi / (h->desc.dx[2] * h->n2);
+  if (h->prec == OPFC_FP64)
+    adj_tables_kernel<<<kEltBlocks, 256, 0, h->stream>>>((double *)h->tab_ar, (double *)h->tab_br, h->M, h->n1, h->n2,
+                                                         h->nyq_off, f0, f1, f2, h->desc.r, h->dt);
+  else
+    adj_tables_kernel<<<kEltBlocks, 256, 0, h->stream>>>((float *)h->tab_ar, (float *)h->tab_br, h->M, h->n1, h->n2,
+                                                         h->nyq_off, f0, f1, f2, h->desc.r, h->dt);
+  CUDA_TRY(h, cudaGetLastError());
   return OPFC_OK;
 }
 
@@ -2342,17 +2352,78 @@ int copy_state(opfc_handle *h, void *dst, const void *src) {
   return OPFC_OK;
 }
 
+// Reverse steps as two kernels (z_adj_kernel, plane_kernel) instead of some
+// twenty: the plain model where the step runs as a plane kernel and the reverse
+// step's three planes fit too.
+bool adj_plane(const opfc_handle *h) {
+  return h->desc.model == OPFC_MODEL_PLAIN && h->plane && plane_fits(h->M, h->n1, (int)h->rsz, kPlaneAdjoint) &&
+         h->n2 >= 32 && h->n2 != 40;
+}
+
 int adjoint_buffers(opfc_handle *h) {
   int rc;
+  const bool plane = adj_plane(h);
   for (auto &p : h->adj_c)
     if (!p && (rc = dev_alloc(h, &p, h->nc * 2 * h->rsz))) return rc;
-  for (auto &p : h->adj_r)
-    if (!p && (rc = dev_alloc(h, &p, h->nr * h->rsz))) return rc;
-  while ((int)h->seg.size() < h->ckpt_K) {
-    void *p = nullptr;
-    if ((rc = dev_alloc(h, &p, h->nc * 2 * h->rsz))) return rc;
-    h->seg.push_back(p);
+  for (int i = 0; i < (plane ? 1 : 4); ++i)
+    if (!h->adj_r[i] && (rc = dev_alloc(h, &h->adj_r[i], h->nr * h->rsz))) return rc;
+  for (auto *v : {&h->seg, &h->seg_a, &h->seg_n}) {
+    if (v != &h->seg && !plane) break;
+    while ((int)v->size() < h->ckpt_K) {
+      void *p = nullptr;
+      if ((rc = dev_alloc(h, &p, h->nc * 2 * h->rsz))) return rc;
+      v->push_back(p);
+    }
   }
+  return OPFC_OK;
+}
+
+// One recomputed step i of a segment of len, kept for adj_plane_step: psi_hat in
+// seg[i], F_z^-1[psi_hat] in seg_a[i] (there already), F_xy[N] in seg_n[i].
+int recompute_plane_step(opfc_handle *h, int i, int len) {
+  int rc;
+  if (i == 0) LAUNCH_TRY(h, col_plain(h, 2, +1, h->psi_hat, h->seg_a[0]));
+  CUDA_TRY(h, cudaMemcpyAsync(h->seg[i], h->psi_hat, h->nc * 2 * h->rsz, cudaMemcpyDeviceToDevice, h->stream));
+  if ((rc = plane_pass(h, h->seg_a[i], h->seg_n[i]))) return rc;
+  if (i + 1 == len) return OPFC_OK;  // the segment's end state is not needed
+  h->z_in = h->seg_n[i];
+  h->z_out = h->seg_a[i + 1];
+  rc = enqueue_step_kernels(h, 3);
+  h->z_in = nullptr;
+  h->z_out = nullptr;
+  return rc ? rc : enqueue_step_kernels(h, 4);
+}
+
+// adj_c[0] <- F_xy of the adjoint of step i, from F_xy[lambda] in adj_c[0]
+int adj_plane_step(opfc_handle *h, int i) {
+  ZAdjArgs z{};
+  z.lam = h->adj_c[0];
+  z.nxy = h->seg_n[i];
+  z.psi_hat = h->seg[i];
+  z.out_a = h->adj_c[0];
+  z.out_b = h->adj_c[1];
+  z.ta = h->tab_a;
+  z.tb = h->tab_b;
+  z.tar = h->tab_ar;
+  z.tbr = h->tab_br;
+  z.tw = h->tw_z;
+  z.M = h->M;
+  z.n1 = h->n1;
+  z.n2 = h->n2;
+  z.nyq_off = h->nyq_off;
+  z.partials = h->partials;
+  z.npartials = h->npartials;
+  const bool f64 = h->prec == OPFC_FP64;
+  LAUNCH_TRY(h, f64 ? launch_z_adj<double>(z, h->stream) : launch_z_adj<float>(z, h->stream));
+  PlaneArgs a = plane_args(h);
+  a.in[0] = h->seg_a[i];
+  a.in[1] = h->adj_c[0];
+  a.in[2] = h->adj_c[1];
+  a.out = h->adj_c[0];
+  a.scale = x_base(h).scale;
+  a.mean_dev = h->mean_dev;
+  LAUNCH_TRY(h, f64 ? launch_plane<double>(kPlaneAdjoint, a, h->stream)
+                    : launch_plane<float>(kPlaneAdjoint, a, h->stream));
   return OPFC_OK;
 }
 
@@ -2432,9 +2503,10 @@ int opfc_set_r(opfc_handle *h, double r) {
   if (!h) return OPFC_ERR_ARG;
   if (two_field(h->desc.model) || user_ops_model(h->desc.model))
     return fail(h, OPFC_ERR_ARG, "r is not a parameter of this model");
+  h->ckpt_steps = 0;
+  if (h->initialized && r == h->desc.r) return OPFC_OK;  // the tables are this r's
   h->desc.r = r;
   release_graph(h);
-  h->ckpt_steps = 0;
   if (h->initialized) return opfc_initialize(h, h->dt);
   return OPFC_OK;
 }
@@ -2478,18 +2550,35 @@ int opfc_adjoint(opfc_handle *h, const void *grad_psi_T, int dtype, int where, v
   CUDA_TRY(h, cudaMemcpyAsync(h->adj_r[0], h->real_buf, h->nr * h->rsz, cudaMemcpyDeviceToDevice, h->stream));
   const int K = h->ckpt_K, n = h->ckpt_steps;
   const int nseg = (n + K - 1) / K;
+  const bool plane = adj_plane(h);
+  if (plane && (rc = xy_forward(h, h->adj_r[0], h->adj_c[0]))) return rc;
   CUDA_TRY(h, cudaMemsetAsync(h->partials, 0, sizeof(double) * h->npartials, h->stream));
   for (int sg = nseg - 1; sg >= 0; --sg) {
     const int len = std::min(K, n - sg * K);
     // recompute the segment's states with the forward step itself
     if ((rc = copy_state(h, h->psi_hat, h->ckpt[sg]))) return rc;
     h->a_valid = false;
+    if (plane) {
+      for (int i = 0; i < len; ++i)
+        if ((rc = recompute_plane_step(h, i, len))) return rc;
+      for (int i = len - 1; i >= 0; --i)
+        if ((rc = adj_plane_step(h, i))) return rc;
+      continue;
+    }
     for (int i = 0; i < len; ++i) {
       if ((rc = copy_state(h, h->seg[i], h->psi_hat))) return rc;
       if ((rc = opfc_step(h, 1))) return rc;
     }
     for (int i = len - 1; i >= 0; --i)
       if ((rc = adjoint_step(h, h->seg[i]))) return rc;
+  }
+  if (plane) {  // F_xy[lambda_0] -> lambda_0: xy_backward scales by 1/(N0 N1 N2)
+    PlaneArgs a = plane_args(h);
+    a.in[0] = h->adj_c[0];
+    a.rout = h->adj_r[0];
+    a.scale = 1.0 / ((double)h->n0 * h->n1);
+    LAUNCH_TRY(h, h->prec == OPFC_FP64 ? launch_plane_fft<double>(+1, a, h->stream)
+                                       : launch_plane_fft<float>(+1, a, h->stream));
   }
   double dr = std::nan("");  // not a parameter of the model
   if (has_r(h)) {

@@ -13,6 +13,11 @@
 // a line as in fft_core.cuh.  The y inverse reads its first stage from HBM into
 // registers and the y forward writes its last stage from registers.
 //
+// Bound by latency (a plane's phases are a serial chain of loads, exchanges and
+// barriers in one CTA), so it pays where the three launches it replaces were
+// short.  A step of 64^3 FP32 went from 16.8 to 11.3 us, of 160x80x96 from 43 to
+// 30 us, of 192x96x80 FP64 from 66 to 50 us (direct-load z update on both sides).
+//
 // The block is as many lines wide as the longer phase needs in equal turns
 // (plane_threads); lines past the end run their barriers idle.
 #pragma once
@@ -205,7 +210,7 @@ __device__ __forceinline__ void plane_x(const PlaneArgs &a, typename Cx<Real>::T
 #pragma unroll 1
     for (int f = 0; f + 1 < NF; ++f) {
       C *row = planes + f * psz + off;
-      plane_x_inverse<Real, C, M>(v, row, tw, j, ok, a.scale, mean);
+      plane_x_inverse<Real, C, M>(v, row, tw, j, ok, a.scale, MODEL == kPlaneAdjoint && f > 0 ? 0.0 : mean);
       if (ok) {
 #pragma unroll
         for (int m = 0; m < E; ++m) row[j + T * m] = v[m];  // read back by this thread only
@@ -213,7 +218,8 @@ __device__ __forceinline__ void plane_x(const PlaneArgs &a, typename Cx<Real>::T
     }
     C *row = planes + (NF - 1) * psz + off;
     // MK_ALUMINUM_G: the last field is P*psi, whose mean is P_F(0) times psi's
-    plane_x_inverse<Real, C, M>(v, row, tw, j, ok, a.scale, MODEL == MK_ALUMINUM_G ? a.al[17] * mean : mean);
+    plane_x_inverse<Real, C, M>(v, row, tw, j, ok, a.scale,
+                                MODEL == MK_ALUMINUM_G ? a.al[17] * mean : MODEL == kPlaneAdjoint ? 0.0 : mean);
     const double time = MODEL == MK_ALUMINUM_G ? *a.time : 0.0;
 #pragma unroll
     for (int m = 0; m < E; ++m) {
@@ -231,6 +237,11 @@ __device__ __forceinline__ void plane_x(const PlaneArgs &a, typename Cx<Real>::T
         const C u = ok ? planes[off + j + T * m] : mk<C>(0, 0);
         nx = c0 * u.x * u.x + c1 * u.x * u.x * u.x + c2 * x * x + c3 * x * x * x - c4 * u.x;
         ny = c0 * u.y * u.y + c1 * u.y * u.y * u.y + c2 * y * y + c3 * y * y * y - c4 * u.y;
+      } else if constexpr (MODEL == kPlaneAdjoint) {
+        const C u = ok ? planes[off + j + T * m] : mk<C>(0, 0);
+        const C g = ok ? planes[psz + off + j + T * m] : mk<C>(0, 0);
+        nx = g.x + Real(3) * u.x * u.x * x;
+        ny = g.y + Real(3) * u.y * u.y * y;
       } else {
         const C u = ok ? planes[off + j + T * m] : mk<C>(0, 0);
         const C w = ok ? planes[psz + off + j + T * m] : mk<C>(0, 0);
@@ -407,7 +418,7 @@ template <typename Real> int launch_plane(int model, const PlaneArgs &a, cudaStr
 #define OPFC_CASE(m) \
   case m: return mixed ? launch_plane_t<Real, m, true>(a, s) : launch_plane_t<Real, m, false>(a, s);
   switch (model) {
-    OPFC_CASE(MK_PLAIN) OPFC_CASE(MK_FILTERED) OPFC_CASE(MK_TUNGSTEN) OPFC_CASE(MK_ALUMINUM_G)
+    OPFC_CASE(MK_PLAIN) OPFC_CASE(MK_FILTERED) OPFC_CASE(MK_TUNGSTEN) OPFC_CASE(MK_ALUMINUM_G) OPFC_CASE(kPlaneAdjoint)
   }
 #undef OPFC_CASE
   return (int)cudaErrorInvalidValue;
@@ -433,7 +444,8 @@ template <typename Real> int launch_plane_fft(int dir, const PlaneArgs &a, cudaS
 // row).  A column is q = kx + (M+1) ky, so W neighbouring columns are W
 // neighbouring values of every reference plane; on the split side the run breaks
 // once a row.  The transform pass does the layout change, which otherwise is a
-// read and a write of the whole spectrum on its own.
+// read and a write of the whole spectrum on its own (256^3 FP64 forward and
+// backward: 543 us with that and the real field's copies, 387 us without).
 // ---------------------------------------------------------------------------
 template <typename Real, int N, int DIR>
 __global__ void __launch_bounds__(Width<Real>::W *(N / Plan<N>::E)) z_ref_kernel(const __grid_constant__ ZRefArgs a) {
@@ -488,6 +500,101 @@ template <typename Real> int launch_z_ref(int dir, const ZRefArgs &a, cudaStream
   case n: return launch_z_ref_n<Real, n>(dir, a, s);
     OPFC_SIZES(OPFC_CASE)
     OPFC_CASE(1)
+#undef OPFC_CASE
+  }
+  return (int)cudaErrorInvalidValue;
+}
+
+// z part of the plain model's reverse step: two forward and two inverse
+// transforms and the mode products in one pass (see ZAdjArgs).  With the plane
+// kernel on (psi, a, w) a reverse step is two launches instead of nineteen; the
+// gradient of 40 steps at 128^3 FP32 went from 28.7 to 6.3 ms with it.
+template <typename Real, int N>
+__global__ void __launch_bounds__(Width<Real>::W *(N / Plan<N>::E)) z_adj_kernel(const __grid_constant__ ZAdjArgs a) {
+  using C = typename Cx<Real>::T;
+  constexpr int W = Width<Real>::W, E = Plan<N>::E, T = N / E, NT = W * T, ld = W + 1;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  C *tw = reinterpret_cast<C *>(smraw);
+  C *sm = tw + N;
+  const int c = threadIdx.x % W, j = threadIdx.x / W;
+  for (int i = threadIdx.x; i < N; i += NT) tw[i] = reinterpret_cast<const C *>(a.tw)[i];
+  const int ti = (a.M + W - 1) / W, mains = ti * a.n1, tiles = mains + (a.n1 + W - 1) / W;
+  const C *lam = reinterpret_cast<const C *>(a.lam), *nxy = reinterpret_cast<const C *>(a.nxy);
+  const C *psi = reinterpret_cast<const C *>(a.psi_hat);
+  C *oa = reinterpret_cast<C *>(a.out_a), *ob = reinterpret_cast<C *>(a.out_b);
+  const Real *ta = reinterpret_cast<const Real *>(a.ta), *tb = reinterpret_cast<const Real *>(a.tb);
+  const Real *tar = reinterpret_cast<const Real *>(a.tar), *tbr = reinterpret_cast<const Real *>(a.tbr);
+  double s = 0;
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const bool nyq = t >= mains;
+    const int cg = (nyq ? t - mains : t % ti) * W + c;
+    const bool ok = cg < (nyq ? a.n1 : a.M);
+    const long long base = nyq ? a.nyq_off + cg : (long long)(t / ti) * a.M + cg;
+    const long long fs = nyq ? a.n1 : (long long)a.M * a.n1;
+    const double wgt = nyq || cg == 0 ? 1.0 : 2.0;
+    C l[E], q[E];
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      l[m] = ok ? lam[base + (j + T * m) * fs] : mk<C>(0, 0);
+      q[m] = ok ? nxy[base + (j + T * m) * fs] : mk<C>(0, 0);
+    }
+    __syncthreads();  // tw; the previous tile's last reads of sm
+    fft_line<C, N, -1, N>(l, sm, ld, c, j, tw);
+    fft_line<C, N, -1, N>(q, sm, ld, c, j, tw);
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      if (ok) {
+        const long long i = base + (j + T * m) * fs;
+        const C p = psi[i];
+        const double ar = tar[i], br = tbr[i];
+        s += wgt * ((double)l[m].x * (ar * p.x + br * q[m].x) + (double)l[m].y * (ar * p.y + br * q[m].y));
+        const Real la = ta[i], lb = tb[i];
+        q[m] = mk<C>(lb * l[m].x, lb * l[m].y);
+        l[m] = mk<C>(la * l[m].x, la * l[m].y);
+      }
+    }
+    fft_line<C, N, +1, N>(l, sm, ld, c, j, tw);
+    fft_line<C, N, +1, N>(q, sm, ld, c, j, tw);
+    if (ok) {
+#pragma unroll
+      for (int m = 0; m < E; ++m) {
+        oa[base + (j + T * m) * fs] = l[m];
+        ob[base + (j + T * m) * fs] = q[m];
+      }
+    }
+  }
+  // block sum in a fixed order (sm holds NT doubles: NT <= N W)
+  double *red = reinterpret_cast<double *>(sm);
+  __syncthreads();
+  red[threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double r = 0;
+    for (int i = threadIdx.x; i < NT; i += 32) r += red[i];
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1) r += __shfl_xor_sync(0xffffffffu, r, h);
+    if (threadIdx.x == 0) a.partials[blockIdx.x] += r;
+  }
+}
+
+template <typename Real, int N> static int launch_z_adj_n(const ZAdjArgs &a, cudaStream_t s) {
+  using C = typename Cx<Real>::T;
+  constexpr int W = Width<Real>::W, NT = W * (N / Plan<N>::E);
+  const size_t smem = sizeof(C) * ((size_t)N + (size_t)N * (W + 1));
+  static int setup[kDevCache];
+  kernel_setup(z_adj_kernel<Real, N>, NT, smem, setup);
+  const int tiles = (a.M + W - 1) / W * a.n1 + (a.n1 + W - 1) / W;
+  z_adj_kernel<Real, N><<<tiles < a.npartials ? tiles : a.npartials, NT, smem, s>>>(a);
+  return (int)cudaGetLastError();
+}
+
+// lengths whose block has a whole warp for the final sum
+template <typename Real> int launch_z_adj(const ZAdjArgs &a, cudaStream_t s) {
+  switch (a.n2) {
+#define OPFC_CASE(n) \
+  case n: return launch_z_adj_n<Real, n>(a, s);
+    OPFC_CASE(32) OPFC_CASE(48) OPFC_CASE(64) OPFC_CASE(80) OPFC_CASE(96) OPFC_CASE(128) OPFC_CASE(256)
+    OPFC_CASE(512) OPFC_CASE(1024)
 #undef OPFC_CASE
   }
   return (int)cudaErrorInvalidValue;

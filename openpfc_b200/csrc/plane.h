@@ -7,9 +7,13 @@
 
 namespace opfc {
 
+// the plain model's reverse step as a plane_kernel "model": fields psi, a, w ->
+// lambda = a + 3 psi^2 w
+constexpr int kPlaneAdjoint = 16;
+
 // real fields of a step, one shared-memory plane each
 constexpr int plane_fields(int model) {
-  return model == MK_TUNGSTEN ? 2 : model == MK_ALUMINUM_G ? 3 : 1;
+  return model == MK_TUNGSTEN ? 2 : model == MK_ALUMINUM_G || model == kPlaneAdjoint ? 3 : 1;
 }
 
 struct PlaneArgs {
@@ -74,5 +78,21 @@ struct ZRefArgs {
   long long nyq_off;
 };
 template <typename Real> int launch_z_ref(int dir, const ZRefArgs &a, cudaStream_t s);
+
+// z part of the plain model's reverse step (split layout): with lambda_hat and
+// N_hat the forward z transforms of lam and nxy,
+//   partials += Re sum w conj(lambda_hat) (tar psi_hat + tbr N_hat)
+//   out_a = F_z^-1[ta lambda_hat] (may be lam), out_b = F_z^-1[tb lambda_hat]
+// (w = 1 on the kx = 0 and kx = M planes, else 2).  At most `npartials` blocks.
+struct ZAdjArgs {
+  const void *lam, *nxy, *psi_hat;
+  void *out_a, *out_b;
+  const void *ta, *tb, *tar, *tbr, *tw;
+  int M, n1, n2;
+  long long nyq_off;
+  double *partials;
+  int npartials;
+};
+template <typename Real> int launch_z_adj(const ZAdjArgs &a, cudaStream_t s);
 
 }  // namespace opfc

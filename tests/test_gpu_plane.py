@@ -96,6 +96,28 @@ def test_transform_device_buffers(oracle, n2, prec):
         assert np.abs(back.double().cpu().numpy() - x).max() <= (1e-12 if prec == ob.FP64 else 2e-6) * np.abs(x).max()
 
 
+@pytest.mark.parametrize("prec,tol", [(ob.FP64, 1e-10), (ob.FP32, 1e-4)])
+@pytest.mark.parametrize("n", [(32, 16, 32), (48, 40, 48), (64, 48, 80)])
+def test_adjoint_against_general_path(monkeypatch, n, prec, tol):
+    """Two kernels a reverse step against the general reverse step (OPFC_PLANE=0):
+    the same sums in another order, over 7 steps with segments of 3, 3 and 1."""
+    psi0 = ob.ic_noise(n, -0.285, 0.05, 8)
+    w = ob.ic_noise(n, 0.0, 1.0, 9)
+    got = []
+    for plane in ("1", "0"):
+        monkeypatch.setenv("OPFC_PLANE", plane)
+        m = ob.PfcB200(n, PI4, r=-0.25, precision=prec)
+        m.initialize(0.5)
+        m.set_psi(psi0)
+        m.forward_checkpointed(7, 3)
+        got.append(m.adjoint(w))
+    (g1, r1, n1), (g0, r0, n0) = got
+    assert _rel(np.asarray(g1), np.asarray(g0)) <= tol
+    # dr and dn0 are sums with cancellation: relative to their terms' size
+    assert abs(r1 - r0) <= tol * max(abs(r0), np.linalg.norm(w) * np.linalg.norm(psi0) * 1e-2)
+    assert abs(n1 - n0) <= tol * max(abs(n0), np.abs(w).sum())
+
+
 @pytest.mark.parametrize("prec", [ob.FP64, ob.FP32])
 def test_ensemble(oracle, prec):
     sides = [(32, 16, 48), (48, 96, 16), (80, 48, 32), (128, 128, 16), (96, 80, 16), (64, 64, 64)]
