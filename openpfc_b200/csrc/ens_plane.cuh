@@ -43,7 +43,7 @@ template <typename Real> __global__ void __launch_bounds__(kEnsPlaneThreads, 2) 
 #undef OPFC_CASE
   __syncthreads();
 #define OPFC_CASE(n) \
-  case n: plane_x<Real, n, MK_PLAIN>(p, plane, 0, twx, bad); break;
+  case n: plane_x<Real, n, MK_PLAIN>(p, plane, 0, twx, nullptr, bad); break;
   switch (M) { OPFC_ENS_PLANE_X(OPFC_CASE) }
 #undef OPFC_CASE
   __syncthreads();

@@ -414,46 +414,6 @@ __global__ void __launch_bounds__(Width<Real>::W *(M / Plan<M>::E)) x_kernel(con
           bad |= !(isfinite(nx) && isfinite(ny));
           v[m] = mk<C>(nx, ny);
         }
-      } else if constexpr (MODEL == MK_ALUMINUM_G) {
-        // Aluminum.hpp:270-307: psi (u), psi_MF (v) and P*psi (q) in real space;
-        // moving temperature T_var(x, t); real cells 2p (re) and 2p + 1 (im)
-        C u[E];
-#pragma unroll
-        for (int m = 0; m < E; ++m) u[m] = v[m];
-        x_load_rows<C, M, W, NT>(reinterpret_cast<const C *>(a.in1), a.nyq_off, row0, a.rows, buf, tid);
-        __syncthreads();
-        x_pre<C, M, W, E>(buf, tw, c, j, v);
-        __syncthreads();
-        fft_line<C, M, +1, N0>(v, buf, ld, c, j, tw);
-        C q[E];
-        x_load_rows<C, M, W, NT>(reinterpret_cast<const C *>(a.in2), a.nyq_off, row0, a.rows, buf, tid);
-        __syncthreads();
-        x_pre<C, M, W, E>(buf, tw, c, j, q);
-        __syncthreads();
-        fft_line<C, M, +1, N0>(q, buf, ld, c, j, tw);
-        const double *al = a.al;
-        const double t = *a.time;
-        auto nl = [&](double x, Real uu, Real vv, Real qq) -> Real {
-          const double dist = x + al[3] - (x > al[4] ? al[2] : 0.0);
-          const double Tv = al[5] * (dist - al[6] - al[7] * t);
-          const Real q2N = (Real)(al[10] * Tv / al[8]);
-          const Real q3 = (Real)(al[12] * (al[9] + Tv) / al[8] + al[11]);
-          const Real kern = (Real)(-(1.0 - exp(-Tv / al[8]))) * qq;
-          return (Real)al[13] * uu * uu + (Real)al[14] * uu * uu * uu + q2N * vv + q3 * vv * vv +
-                 (Real)al[15] * vv * vv * vv - kern - (Real)al[16] * uu;
-        };
-#pragma unroll
-        for (int m = 0; m < E; ++m) {
-          const Real vx = to_real_plus_mean(v[m].x, a.scale, a.mean);
-          const Real vy = to_real_plus_mean(v[m].y, a.scale, a.mean);
-          const Real qx = to_real_plus_mean(q[m].x, a.scale, al[17] * a.mean);
-          const Real qy = to_real_plus_mean(q[m].y, a.scale, al[17] * a.mean);
-          const int i0 = 2 * (j + T * m);
-          const Real nx = nl(al[0] + i0 * al[1], u[m].x, vx, qx);
-          const Real ny = nl(al[0] + (i0 + 1) * al[1], u[m].y, vy, qy);
-          bad |= !(isfinite(nx) && isfinite(ny));
-          v[m] = mk<C>(nx, ny);
-        }
       } else if constexpr (MODEL == MK_FILTERED) {
         // N = p2 v^2/2 + p3 v^3/3 + p4 v^4/4 of the filtered density
 #pragma unroll
@@ -1029,7 +989,6 @@ static int launch_x_m(const XLaunch &L, cudaStream_t s) {
     case MK_PLAIN: return launch_x_t<Real, M, X_FUSED, MK_PLAIN>(L, s);
     case MK_TUNGSTEN: return launch_x_t<Real, M, X_FUSED, MK_TUNGSTEN>(L, s);
     case MK_FILTERED: return launch_x_t<Real, M, X_FUSED, MK_FILTERED>(L, s);
-    case MK_ALUMINUM_G: return launch_x_t<Real, M, X_FUSED, MK_ALUMINUM_G>(L, s);
   }
   return (int)cudaErrorInvalidValue;
 }

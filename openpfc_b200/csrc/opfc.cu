@@ -317,6 +317,9 @@ int col(opfc_handle *h, ColLaunch L) {
   return h->prec == OPFC_FP64 ? launch_col<double>(L, h->stream) : launch_col<float>(L, h->stream);
 }
 int xpass(opfc_handle *h, const XLaunch &L) {
+  if (L.mode == X_FUSED && L.model == MK_ALUMINUM_G)
+    return h->prec == OPFC_FP64 ? launch_al_x<double>(L, h->mean_dev, h->stream)
+                                : launch_al_x<float>(L, h->mean_dev, h->stream);
   return h->prec == OPFC_FP64 ? launch_x<double>(L, h->stream) : launch_x<float>(L, h->stream);
 }
 
@@ -787,7 +790,7 @@ int enqueue_steps(opfc_handle *h, int n) {
 
 // Whether the captured step outlives the field: these x passes read the mean
 // density from device memory; the others take it as a launch argument.
-bool keeps_graph(const opfc_handle *h) { return h->plane; }
+bool keeps_graph(const opfc_handle *h) { return h->plane || h->al_grad; }
 
 // Steps of one graph: a small grid's step is a few short kernels, so the gap
 // between graph launches would be a good part of it.

@@ -21,7 +21,7 @@
 // The block is as many lines wide as the longer phase needs in equal turns
 // (plane_threads); lines past the end run their barriers idle.
 #pragma once
-#include "kernels.cuh"
+#include "aluminum.cuh"
 #include "plane.h"
 
 namespace opfc {
@@ -150,17 +150,6 @@ __device__ __forceinline__ void plane_x_inverse(C (&v)[Plan<M>::E], C *row, cons
     v[m] = mk<C>(to_real_plus_mean(v[m].x, scale, mean), to_real_plus_mean(v[m].y, scale, mean));
 }
 
-// Aluminum nonlinearity at position x and time t (Aluminum.hpp:270-307; al as XLaunch::al)
-template <typename Real> __device__ __forceinline__ Real aluminum_nl(const double *al, double t, double x, Real u, Real v, Real q) {
-  const double dist = x + al[3] - (x > al[4] ? al[2] : 0.0);
-  const double Tv = al[5] * (dist - al[6] - al[7] * t);
-  const Real q2N = (Real)(al[10] * Tv / al[8]);
-  const Real q3 = (Real)(al[12] * (al[9] + Tv) / al[8] + al[11]);
-  const Real kern = (Real)(-(1.0 - exp(-Tv / al[8]))) * q;
-  return (Real)al[13] * u * u + (Real)al[14] * u * u * u + q2N * v + q3 * v * v + (Real)al[15] * v * v * v - kern -
-         (Real)al[16] * u;
-}
-
 // R2C of one row held in registers; the spectrum (modes 0..M) replaces the row
 template <typename Real, typename C, int M>
 __device__ __forceinline__ void plane_x_forward(C (&v)[Plan<M>::E], C *row, const C *tw, int j, bool ok) {
@@ -195,7 +184,7 @@ __device__ __forceinline__ void plane_x_forward(C (&v)[Plan<M>::E], C *row, cons
 // the last field's plane.  The earlier fields' real values wait in their own rows.
 template <typename Real, int M, int MODEL>
 __device__ __forceinline__ void plane_x(const PlaneArgs &a, typename Cx<Real>::T *planes, size_t psz,
-                                        const typename Cx<Real>::T *tw, bool &bad) {
+                                        const typename Cx<Real>::T *tw, const AlCoef<Real> *coef, bool &bad) {
   using C = typename Cx<Real>::T;
   constexpr int E = Plan<M>::E, T = M / E, P = M + 1;
   constexpr int NF = plane_fields(MODEL);
@@ -220,7 +209,6 @@ __device__ __forceinline__ void plane_x(const PlaneArgs &a, typename Cx<Real>::T
     // MK_ALUMINUM_G: the last field is P*psi, whose mean is P_F(0) times psi's
     plane_x_inverse<Real, C, M>(v, row, tw, j, ok, a.scale,
                                 MODEL == MK_ALUMINUM_G ? a.al[17] * mean : MODEL == kPlaneAdjoint ? 0.0 : mean);
-    const double time = MODEL == MK_ALUMINUM_G ? *a.time : 0.0;
 #pragma unroll
     for (int m = 0; m < E; ++m) {
       const Real x = v[m].x, y = v[m].y;
@@ -246,8 +234,8 @@ __device__ __forceinline__ void plane_x(const PlaneArgs &a, typename Cx<Real>::T
         const C u = ok ? planes[off + j + T * m] : mk<C>(0, 0);
         const C w = ok ? planes[psz + off + j + T * m] : mk<C>(0, 0);
         const int i0 = 2 * (j + T * m);
-        nx = aluminum_nl<Real>(a.al, time, a.al[0] + i0 * a.al[1], u.x, w.x, x);
-        ny = aluminum_nl<Real>(a.al, time, a.al[0] + (i0 + 1) * a.al[1], u.y, w.y, y);
+        nx = aluminum_nl<Real>(a.al, coef[i0], u.x, w.x, x);
+        ny = aluminum_nl<Real>(a.al, coef[i0 + 1], u.y, w.y, y);
       }
       bad |= ok && !(isfinite(nx) && isfinite(ny));
       v[m] = mk<C>(nx, ny);
@@ -328,6 +316,12 @@ __global__ void __launch_bounds__(kPlaneThreads<Real>, kPlaneCtas<Real, MIXED>)
   __syncthreads();
   const long long main0 = (long long)blockIdx.x * M * n1, nyq0 = a.nyq_off + (long long)blockIdx.x * n1;
   bool bad = false;
+  AlCoef<Real> *coef = nullptr;  // MK_ALUMINUM_G: per x position (visible after the y phase's barrier)
+  if constexpr (MODEL == MK_ALUMINUM_G) {
+    coef = reinterpret_cast<AlCoef<Real> *>(planes + NF * psz);
+    const double t = *a.time;
+    for (int i = threadIdx.x; i < n0; i += blockDim.x) coef[i] = aluminum_coef<Real>(a.al, t, a.al[0] + i * a.al[1]);
+  }
 #pragma unroll 1
   for (int f = 0; f < NF; ++f) {
     const C *in = reinterpret_cast<const C *>(a.in[f]);
@@ -338,7 +332,7 @@ __global__ void __launch_bounds__(kPlaneThreads<Real>, kPlaneCtas<Real, MIXED>)
   }
   __syncthreads();
 #define OPFC_CASE(n) \
-  case n: plane_x<Real, n, MODEL>(a, planes, psz, twx, bad); break;
+  case n: plane_x<Real, n, MODEL>(a, planes, psz, twx, coef, bad); break;
   OPFC_PLANE_SWITCH(M, OPFC_CASE)
 #undef OPFC_CASE
   __syncthreads();

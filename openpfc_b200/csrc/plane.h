@@ -45,7 +45,8 @@ constexpr bool plane_len_ok(int N) {
          N == 256 || N == 512;
 }
 constexpr size_t plane_smem(int M, int n1, int rsz, int model) {
-  return (size_t)2 * rsz * (n1 + 2 * (size_t)M + (size_t)plane_fields(model) * (M + 1) * n1);
+  return (size_t)2 * rsz * (n1 + 2 * (size_t)M + (size_t)plane_fields(model) * (M + 1) * n1) +
+         (model == MK_ALUMINUM_G ? (size_t)3 * rsz * 2 * M : 0);  // temperature coefficients per x position
 }
 constexpr bool plane_fits(int M, int n1, int rsz, int model) {
   return plane_len_ok(M) && plane_len_ok(n1) && plane_smem(M, n1, rsz, model) <= 232448;
@@ -67,6 +68,9 @@ inline int plane_threads(int M, int n1, int rsz) {
 template <typename Real> int launch_plane(int model, const PlaneArgs &a, cudaStream_t s);
 // dir < 0: rin -> x R2C, y forward -> out; dir > 0: in[0] -> y inverse, x C2R -> rout
 template <typename Real> int launch_plane_fft(int dir, const PlaneArgs &a, cudaStream_t s);
+
+// Fused x pass of MK_ALUMINUM_G, mean density from device memory (aluminum_f32.cu / aluminum_f64.cu)
+template <typename Real> int launch_al_x(const XLaunch &L, const double *mean_dev, cudaStream_t s);
 
 // z transform of a whole spectrum, split layout -> reference layout (dir < 0)
 // or back (dir > 0)
