@@ -13,6 +13,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <system_error>
 #include <thread>
@@ -89,13 +90,17 @@ class HostPipe {
     for (cudaEvent_t e : ev_)
       if (e) cudaEventDestroy(e);
     ev_.clear();
-    if (pin_) cudaFreeHost(pin_);
+    if (pin_ && pinned_)
+      cudaFreeHost(pin_);
+    else
+      std::free(pin_);
     pin_ = nullptr;
     threads_ = 0;
   }
 
  private:
   char *pin_ = nullptr;
+  bool pinned_ = false;  // else pageable: the copies are then slower and synchronous, with the same result
   int threads_ = 0;  // threads with slots and events
   std::vector<cudaEvent_t> ev_;
 
@@ -111,10 +116,10 @@ class HostPipe {
     for (cudaEvent_t e : ev_) cudaEventSynchronize(e);  // copies out of the old slots
     release();
     cudaError_t e = cudaHostAlloc((void **)&pin_, 2 * kSlotBytes * threads, cudaHostAllocDefault);
-    if (e != cudaSuccess) {
+    pinned_ = e == cudaSuccess;
+    if (!pinned_) {
       cudaGetLastError();
-      pin_ = nullptr;
-      return e;
+      if (!(pin_ = static_cast<char *>(std::malloc(2 * kSlotBytes * threads)))) return e;
     }
     for (int i = 0; i < 2 * threads; ++i) {
       cudaEvent_t v = nullptr;

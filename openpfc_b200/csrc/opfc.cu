@@ -161,6 +161,7 @@ struct opfc_handle {
   // plane-kernel adjoint of the plain model: each step's F_z^-1[psi_hat] and
   // F_xy[N] of the recomputed segment, and the z update's arrays meanwhile
   std::vector<void *> seg_a, seg_n;
+  bool no_adj_plane = false;  // no memory for them: the general reverse step
   const void *z_in = nullptr;
   void *z_out = nullptr;
   void *adj_c[2] = {nullptr, nullptr};
@@ -2359,7 +2360,7 @@ int copy_state(opfc_handle *h, void *dst, const void *src) {
 // twenty: the plain model where the step runs as a plane kernel and the reverse
 // step's three planes fit too.
 bool adj_plane(const opfc_handle *h) {
-  return h->desc.model == OPFC_MODEL_PLAIN && h->plane && plane_fits(h->M, h->n1, (int)h->rsz, kPlaneAdjoint) &&
+  return h->desc.model == OPFC_MODEL_PLAIN && h->plane && !h->no_adj_plane && plane_fits(h->M, h->n1, (int)h->rsz, kPlaneAdjoint) &&
          h->n2 >= 32 && h->n2 != 40;
 }
 
@@ -2374,7 +2375,16 @@ int adjoint_buffers(opfc_handle *h) {
     if (v != &h->seg && !plane) break;
     while ((int)v->size() < h->ckpt_K) {
       void *p = nullptr;
-      if ((rc = dev_alloc(h, &p, h->nc * 2 * h->rsz))) return rc;
+      if ((rc = dev_alloc(h, &p, h->nc * 2 * h->rsz))) {
+        if (v == &h->seg || rc != OPFC_ERR_OOM) return rc;
+        for (auto *w : {&h->seg_a, &h->seg_n}) {
+          for (void *q : *w) cudaFree(q);
+          h->allocated -= w->size() * h->nc * 2 * h->rsz;
+          w->clear();
+        }
+        h->no_adj_plane = true;
+        return adjoint_buffers(h);
+      }
       v->push_back(p);
     }
   }
