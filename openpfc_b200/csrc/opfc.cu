@@ -616,13 +616,28 @@ XLaunch x_fused(opfc_handle *h) {
 bool plane_ok(const opfc_handle *h) {
   return plane_fits(h->M, h->n1, (int)h->rsz, x_fused(const_cast<opfc_handle *>(h)).model);
 }
-bool plane_default(const opfc_handle *h) { return h->use_tma && plane_ok(h); }
+// One CTA carries a plane, so few planes leave most of the chip idle: the plane
+// kernel wins up to about 150 modes (of all fields together) per plane and kz
+// plane.  On large grids the separate passes come close to the memory's rate,
+// and one or two latency-bound CTAs per SM do not: it stops at 2^22 cells of all
+// fields.  Measured per step, separate passes / plane kernel (us): 64x64x24
+// FP32 20.8 / 15.2, 128x128x128 42.5 / 39.1, 192x96x80 47 / 35, 128x256x128
+// 59 / 50, 256x48x256 FP64 73 / 68, but 128x128x32 FP32 20.8 / 23.3,
+// 256x128x16 21 / 39, 1024x48x64 54 / 66, 256x128x256 98 / 106, 96x96x1024 FP64
+// 240 / 255; Tungsten 160x80x96 FP64 78 / 58, 96x80x48 32.5 / 36.6, 128x96x256
+// FP32 63 / 71.
+bool plane_pays(const opfc_handle *h, int fields) {
+  return fields * (h->M + 1) * h->n1 <= 150 * h->n2 && fields * h->nr <= ((size_t)1 << 22);
+}
+bool plane_default(const opfc_handle *h) {
+  return h->use_tma && plane_ok(h) && plane_pays(h, plane_fields(x_fused(const_cast<opfc_handle *>(h)).model));
+}
 
 // The transform's plane kernel: where it fits and no pass is forced.
 bool plane_fft_default(const opfc_handle *h) {
   const char *pv = std::getenv("OPFC_PLANE");
   return h->use_tma && plane_fits(h->M, h->n1, (int)h->rsz, MK_PLAIN) && !std::getenv("OPFC_Y_VARIANT") &&
-         !std::getenv("OPFC_X_VARIANT") && !(pv && std::atoi(pv) != 1);
+         !std::getenv("OPFC_X_VARIANT") && (pv ? std::atoi(pv) == 1 : plane_pays(h, 1));
 }
 
 // the step's plane kernel, work_a in place unless told otherwise
@@ -904,6 +919,49 @@ int user_sum(opfc_handle *h, const void *src, int dtype, double *out) {
 bool direct_ok(const opfc_handle *h, const void *p, int dtype, int where) {
   return where == OPFC_DEVICE && (dtype == OPFC_F64) == (h->prec == OPFC_FP64) &&
          reinterpret_cast<uintptr_t>(p) % (2 * h->rsz) == 0;
+}
+
+// Variants of the passes when neither the autotuner nor the environment chose
+// (us a step, the other passes alike).
+bool pow2(int n) { return (n & (n - 1)) == 0; }
+
+// Direct loads on short lines: the pipelined kernel keeps one CTA per SM, with
+// 20 or 24 values a thread on mixed lengths.  512x96x256 FP64 pipelined 351,
+// direct 265; 256^3 FP64 339 / 325; 256x256x128 FP32 108 / 103; but 256x256x512
+// FP32 311 / 323 and 512^3 FP32 1142 / 1365.  Of the pipelined kernels the
+// ping-pong one: 512^3 FP32 1298 (y variant 0) / 1280, 256x256x1024 725 / 711.
+int default_y(const opfc_handle *h) {
+  if (!pow2(h->n1)) return 1;
+  const bool shorter = h->n1 <= 256 && (h->prec == OPFC_FP64 || h->nr < ((size_t)1 << 25));
+  return shorter ? 1 : 3;
+}
+
+// Rows loaded straight into registers from 2^26 cells on at M = 256, FP32 (512^3:
+// 1142 staged, 1130); below that the staged rows win (256x256x512 311 / 326).
+int default_x(const opfc_handle *h) {
+  return h->M == 256 && h->prec == OPFC_FP32 && h->nr >= ((size_t)1 << 26) ? 3 : 0;
+}
+
+// Folded tables (each read once for two tiles) in place of the streamed ones.
+// - Direct loads up to 128 points and on mixed lengths (64x512x96 FP32 pipelined
+//   102, direct 79; 192x96x80 FP64 101 / 66; 256x256x128 FP32 108 / 99;
+//   512x256x128 FP64 366 / 330), and on small grids up to 512 points (64x64x512
+//   FP32 43 / 39); from 2^25 cells on the pipelined kernel (equal at 2^24:
+//   512x256x128 FP32 185 / 185).
+// - At 256 points with ping-pong buffers, longer without: 256^3 FP64 337 with,
+//   339 without, Tungsten 488 / 497; 512^3 FP32 1167 / 1142, filtered
+//   256x128x512 FP64 403 / 354.
+// - Rows of 128 bytes at 1024 points where the kz planes are a megabyte or more
+//   apart (1024^3 filtered: 5.4 ms the pass, 64-byte rows 7.7); at 256 KB they
+//   lose (filtered 256x256x1024: 719 / 704).
+int default_z(const opfc_handle *h) {
+  if (!h->fold_ops || h->slab) return 0;
+  if (!pow2(h->n2) || (h->n2 <= 128 && h->nr < ((size_t)1 << 25)) ||
+      (h->n2 <= 512 && h->nr < ((size_t)1 << 22)))
+    return 7;
+  if (h->n2 <= 256) return 6;
+  const bool one_field = h->desc.model == OPFC_MODEL_PLAIN || h->desc.model == OPFC_MODEL_FILTERED;
+  return h->n2 == 1024 && one_field && (size_t)h->M * h->n1 * 2 * h->rsz >= ((size_t)1 << 20) ? 9 : 8;
 }
 
 // real rows -> dst: x R2C, y forward
@@ -1261,6 +1319,7 @@ int opfc_create(const opfc_desc *d, opfc_handle **out) {
     hp->num_sms = 148;
   hp->tmaps.reserve(64);
   hp->plane_fft = plane_fft_default(hp);
+  hp->var_y = default_y(hp);
   *out = h.release();
   return OPFC_OK;
 }
@@ -1493,9 +1552,9 @@ static int finish_initialize(opfc_handle *h) {
   const int model = h->desc.model;
   // kernel variants: the autotuner's cached choice, else the defaults;
   // OPFC_Y_VARIANT / OPFC_X_VARIANT / OPFC_Z_VARIANT force a pass's variant
-  h->var_y = AutoTuner::instance().get_config(tune_key(h, "y"), 0);
-  h->var_x = AutoTuner::instance().get_config(tune_key(h, "x"), 0);
-  h->var_z = AutoTuner::instance().get_config(tune_key(h, "z"), 0);
+  h->var_y = AutoTuner::instance().get_config(tune_key(h, "y"), default_y(h));
+  h->var_x = AutoTuner::instance().get_config(tune_key(h, "x"), default_x(h));
+  h->var_z = AutoTuner::instance().get_config(tune_key(h, "z"), default_z(h));
   // a cached FP32 choice with per-mode FP32 operators needs the opt-in
   if (z_computed(h->var_z) && h->prec == OPFC_FP32 && !computed_ops_allowed()) h->var_z = h->fold_ops ? 6 : 0;
   if (const char *zv = std::getenv("OPFC_Z_VARIANT")) h->var_z = std::atoi(zv);
