@@ -161,6 +161,7 @@ struct opfc_handle {
   // plane-kernel adjoint of the plain model: each step's F_z^-1[psi_hat] and
   // F_xy[N] of the recomputed segment, and the z update's arrays meanwhile
   std::vector<void *> seg_a, seg_n;
+  std::vector<DevBuf> seg_block[3];  // the allocations behind seg, seg_a, seg_n
   bool no_adj_plane = false;  // no memory for them: the general reverse step
   const void *z_in = nullptr;
   void *z_out = nullptr;
@@ -1227,9 +1228,8 @@ int opfc_destroy(opfc_handle *h) {
     if (p) cudaFree(p);
   for (void *p : h->ckpt)
     if (p) cudaFree(p);
-  for (auto *v : {&h->seg, &h->seg_a, &h->seg_n})
-    for (void *p : *v)
-      if (p) cudaFree(p);
+  for (const auto &v : h->seg_block)
+    for (const DevBuf &b : v) cudaFree(b.p);
   void *adj[] = {h->tab_ar,   h->tab_br,   h->adj_c[0], h->adj_c[1], h->adj_r[0], h->adj_r[1],
                  h->adj_r[2], h->adj_r[3], h->rad_ops,  h->rad_chi,  h->tab_p,    h->work_c,
                  h->time_dev, h->fold_ops, h->fold_chi};
@@ -1319,7 +1319,6 @@ int opfc_create(const opfc_desc *d, opfc_handle **out) {
     hp->num_sms = 148;
   hp->tmaps.reserve(64);
   hp->plane_fft = plane_fft_default(hp);
-  hp->var_y = default_y(hp);
   *out = h.release();
   return OPFC_OK;
 }
@@ -2430,22 +2429,30 @@ int adjoint_buffers(opfc_handle *h) {
     if (!p && (rc = dev_alloc(h, &p, h->nc * 2 * h->rsz))) return rc;
   for (int i = 0; i < (plane ? 1 : 4); ++i)
     if (!h->adj_r[i] && (rc = dev_alloc(h, &h->adj_r[i], h->nr * h->rsz))) return rc;
-  for (auto *v : {&h->seg, &h->seg_a, &h->seg_n}) {
-    if (v != &h->seg && !plane) break;
-    while ((int)v->size() < h->ckpt_K) {
-      void *p = nullptr;
-      if ((rc = dev_alloc(h, &p, h->nc * 2 * h->rsz))) {
-        if (v == &h->seg || rc != OPFC_ERR_OOM) return rc;
-        for (auto *w : {&h->seg_a, &h->seg_n}) {
-          for (void *q : *w) cudaFree(q);
-          h->allocated -= w->size() * h->nc * 2 * h->rsz;
-          w->clear();
+  // one allocation for all missing steps of a kind (every cudaMalloc of a
+  // handle's first gradient counts), each step's array on its own 256 bytes
+  const size_t bytes = (h->nc * 2 * h->rsz + 255) / 256 * 256;
+  std::vector<void *> *kind[3] = {&h->seg, &h->seg_a, &h->seg_n};
+  for (int k = 0; k < (plane ? 3 : 1); ++k) {
+    const int missing = h->ckpt_K - (int)kind[k]->size();
+    if (missing <= 0) continue;
+    DevBuf b;
+    b.bytes = bytes * missing;
+    if ((rc = dev_alloc(h, &b.p, b.bytes))) {
+      if (k == 0 || rc != OPFC_ERR_OOM) return rc;
+      for (int q = 1; q < 3; ++q) {
+        for (const DevBuf &f : h->seg_block[q]) {
+          cudaFree(f.p);
+          h->allocated -= f.bytes;
         }
-        h->no_adj_plane = true;
-        return adjoint_buffers(h);
+        h->seg_block[q].clear();
+        kind[q]->clear();
       }
-      v->push_back(p);
+      h->no_adj_plane = true;
+      return adjoint_buffers(h);
     }
+    h->seg_block[k].push_back(b);
+    for (int i = 0; i < missing; ++i) kind[k]->push_back(static_cast<char *>(b.p) + bytes * i);
   }
   return OPFC_OK;
 }
