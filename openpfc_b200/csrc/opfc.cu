@@ -1314,6 +1314,9 @@ int opfc_create(const opfc_desc *d, opfc_handle **out) {
   if ((rc = dev_alloc(hp, (void **)&hp->partials, sizeof(double) * (hp->npartials + 1)))) return cleanup(rc);
   hp->mean_dev = hp->partials + hp->npartials;
   if (cudaMemset(hp->flag, 0, sizeof(unsigned int)) != cudaSuccess) return cleanup(OPFC_ERR_CUDA);
+  // a field that comes through opfc_pass keeps its mean in psi_hat: 0 is added
+  // to it until opfc_set_psi says otherwise
+  if (cudaMemsetAsync(hp->mean_dev, 0, sizeof(double), hp->stream) != cudaSuccess) return cleanup(OPFC_ERR_CUDA);
   if (cudaMemset(hp->psi_hat, 0, cb) != cudaSuccess) return cleanup(OPFC_ERR_CUDA);
   if (cudaDeviceGetAttribute(&hp->num_sms, cudaDevAttrMultiProcessorCount, hp->device) != cudaSuccess)
     hp->num_sms = 148;

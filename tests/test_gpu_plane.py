@@ -131,3 +131,32 @@ def test_ensemble(oracle, prec):
     e.sync()
     for i, p in enumerate(psi):
         assert _rel(e.get_psi(i), oracle.run_plain(p, PI4, ms[i]["r"], 0.5, 10)) <= TOL[prec]
+
+
+@pytest.mark.parametrize("plane", ["1", "0"])
+@pytest.mark.parametrize("prec", [ob.FP64, ob.FP32])
+def test_field_through_passes(oracle, monkeypatch, plane, prec):
+    """A field that came through opfc_pass keeps its mean in psi_hat, so the steps
+    add none: also where the handle's memory held another handle's mean before."""
+    import torch
+
+    from openpfc_b200.sharded import ARRAY_REAL, PASS_XY_FORWARD, PASS_Z_FORWARD, _CudaArray
+
+    monkeypatch.setenv("OPFC_PLANE", plane)
+    n = (32, 16, 48)
+    psi0 = ob.ic_noise(n, -0.285, 0.01, 14)
+    before = ob.PfcB200(n, PI4, r=-0.25, precision=prec)
+    before.initialize(0.5)
+    before.set_psi(ob.ic_noise(n, 0.7, 0.01, 15))
+    before.close()
+    m = ob.PfcB200(n, PI4, r=-0.25, precision=prec)
+    m.initialize(0.5)
+    ptr = ob.lib().opfc_array(m.handle, ARRAY_REAL)
+    real = torch.as_tensor(_CudaArray(ptr, m.shape, "<f8" if prec == ob.FP64 else "<f4"), device="cuda")
+    real.copy_(torch.from_numpy(psi0))
+    torch.cuda.synchronize()
+    for p in (PASS_XY_FORWARD, PASS_Z_FORWARD):
+        assert ob.lib().opfc_pass(m.handle, p, 0.0, 0) == 0
+    m.step(3)
+    m.sync()
+    assert _rel(m.get_psi(), oracle.run_plain(psi0, PI4, -0.25, 0.5, 3)) <= TOL[prec]
