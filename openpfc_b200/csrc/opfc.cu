@@ -223,10 +223,14 @@ int fail(opfc_handle *h, int code, const char *fmt, ...) {
   return code;
 }
 
+// (the error is reported here: the next launch's check does not report it again)
 #define CUDA_TRY(h, expr)                                                                 \
   do {                                                                                    \
     cudaError_t e_ = (expr);                                                              \
-    if (e_ != cudaSuccess) return fail(h, OPFC_ERR_CUDA, "%s: %s", #expr, cudaGetErrorString(e_)); \
+    if (e_ != cudaSuccess) {                                                              \
+      cudaGetLastError();                                                                 \
+      return fail(h, OPFC_ERR_CUDA, "%s: %s", #expr, cudaGetErrorString(e_));             \
+    }                                                                                     \
   } while (0)
 
 #define LAUNCH_TRY(h, expr)                                                                \
@@ -1331,6 +1335,9 @@ static int finish_initialize(opfc_handle *h);
 int opfc_initialize(opfc_handle *h, double dt) {
   if (!h) return OPFC_ERR_ARG;
   if (!(dt > 0) || !std::isfinite(dt)) return fail(h, OPFC_ERR_ARG, "dt must be positive and finite");
+  // a call that fails on the way leaves tables of two kinds or none: no step
+  // uses them until a later call has gone through
+  h->initialized = false;
   CUDA_TRY(h, cudaSetDevice(h->device));
   if (user_ops_model(h->desc.model)) {  // the caller's tables already include dt
     if (!h->user_ops) return fail(h, OPFC_ERR_STATE, "user ETD model: call opfc_set_operators first");
@@ -2589,7 +2596,7 @@ int opfc_set_r(opfc_handle *h, double r) {
   if (h->initialized && r == h->desc.r) return OPFC_OK;  // the tables are this r's
   h->desc.r = r;
   release_graph(h);
-  if (h->initialized) return opfc_initialize(h, h->dt);
+  if (h->dt > 0) return opfc_initialize(h, h->dt);  // tables were built, or half built by a call that failed
   return OPFC_OK;
 }
 
@@ -2624,6 +2631,7 @@ int opfc_adjoint(opfc_handle *h, const void *grad_psi_T, int dtype, int where, v
   int rc;
   if ((rc = check_dtype_where(h, dtype, where))) return rc;
   if (h->ckpt_steps < 1) return fail(h, OPFC_ERR_STATE, "run opfc_forward_checkpointed first");
+  if (!h->initialized) return fail(h, OPFC_ERR_STATE, "opfc_adjoint needs the operator tables");
   CUDA_TRY(h, cudaSetDevice(h->device));
   if ((rc = adjoint_tables(h))) return rc;  // r or dt may have changed since the last call
   if ((rc = adjoint_buffers(h))) return rc;

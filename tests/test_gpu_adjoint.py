@@ -89,3 +89,38 @@ def test_autograd_function_matches_adjoint():
     g, gr, _ = adjoint(n, psi0.detach().cpu().numpy(), -0.25, 20, 5, target.cpu().numpy(), ob.FP64)
     np.testing.assert_allclose(psi0.grad.cpu().numpy(), g, rtol=1e-10, atol=1e-14)
     assert abs(float(r.grad) - gr) <= 1e-10 * abs(gr)
+
+
+def test_set_r_after_a_failed_rebuild(oracle):
+    """A rebuild of the tables that fails (here: its synchronous copies are refused
+    while a stream capture is open) leaves no tables to step with, and the same r
+    given again builds them."""
+    import torch
+
+    n = (32, 32, 32)
+    psi0 = ob.ic_noise(n, -0.285, 0.01, 6)
+    m = ob.PfcB200(n, PI4, r=-0.25, precision=ob.FP64)
+    m.initialize(DT)
+    m.set_psi(psi0)
+    x = torch.zeros(8, device="cuda")
+    torch.cuda.synchronize()
+    failed = None
+    try:
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            x += 1
+            try:
+                m.set_r(-0.3)
+            except ob.OpfcError as e:
+                failed = e
+    except RuntimeError:  # the refused call ends the capture
+        pass
+    torch.cuda.synchronize()
+    assert failed is not None
+    with pytest.raises(ob.OpfcError):
+        m.step(1)
+    m.set_r(-0.3)
+    m.set_psi(psi0)
+    m.step(5)
+    m.sync()
+    ref = oracle.run_plain(psi0, PI4, -0.3, DT, 5)
+    assert np.linalg.norm((m.get_psi() - ref).ravel()) <= 1e-11 * np.linalg.norm(ref.ravel())
