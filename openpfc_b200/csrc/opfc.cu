@@ -31,6 +31,7 @@
 #include "launch.h"
 #include "plane.h"
 #include "twiddle.h"
+#include "user_buffer.h"
 #include "autotune.h"
 #include "io.h"
 
@@ -918,12 +919,13 @@ int user_sum(opfc_handle *h, const void *src, int dtype, double *out) {
   return OPFC_OK;
 }
 
-// Whether `p` can stand in for real_buf or a spectrum buffer in the passes: a
-// device array of the compute precision on a complex value's boundary (the
-// kernels move real rows as (x[2p], x[2p+1]) pairs).
+// Whether `p` can stand in for real_buf or a spectrum buffer in the passes: an
+// array of the compute precision in the handle's own device memory, on a complex
+// value's boundary (the kernels move real rows as (x[2p], x[2p+1]) pairs).
+// Everything else is copied, which also reaches other GPUs' memory.
 bool direct_ok(const opfc_handle *h, const void *p, int dtype, int where) {
   return where == OPFC_DEVICE && (dtype == OPFC_F64) == (h->prec == OPFC_FP64) &&
-         reinterpret_cast<uintptr_t>(p) % (2 * h->rsz) == 0;
+         reinterpret_cast<uintptr_t>(p) % (2 * h->rsz) == 0 && own_device_memory(pointer_attributes(p), h->device);
 }
 
 // Variants of the passes when neither the autotuner nor the environment chose
@@ -1596,16 +1598,16 @@ int opfc_set_psi(opfc_handle *h, const void *psi, size_t count, int dtype, int w
   const bool direct = direct_ok(h, psi, dtype, where);
   // k = 0 mode in FP64 with compensated summation of the caller's values in
   // their own precision (before any rounding to the compute precision).  A
-  // host field already in the compute precision arrives bit for bit in the
-  // device buffer, so its sum runs there; another one is summed by the host
-  // threads that convert it.
+  // field already in the compute precision arrives bit for bit in the device
+  // buffer, so its sum runs there; a host field that is not is summed by the
+  // host threads that convert it.
   const bool same_prec = (dtype == OPFC_F64) == (h->prec == OPFC_FP64);
   const bool host_sum = where == OPFC_HOST && !same_prec;
   std::vector<double> parts;
   if (!direct && (rc = real_in(h, psi, dtype, where, host_sum ? &parts : nullptr))) return rc;
   if (host_sum)
     h->mass_sum = neumaier(parts.data(), parts.size());
-  else if ((rc = user_sum(h, where == OPFC_HOST ? h->real_buf : psi, dtype, &h->mass_sum)))
+  else if ((rc = user_sum(h, same_prec && !direct ? h->real_buf : psi, dtype, &h->mass_sum)))
     return rc;
   if ((rc = forward_real(h, direct ? psi : h->real_buf, h->psi_hat))) return rc;
   // the DC slot of the FP32/FP64 array stays zero; mass_sum carries it
