@@ -237,7 +237,8 @@ __device__ __forceinline__ void plane_x(const PlaneArgs &a, typename Cx<Real>::T
         nx = aluminum_nl<Real>(a.al, coef[i0], u.x, w.x, x);
         ny = aluminum_nl<Real>(a.al, coef[i0 + 1], u.y, w.y, y);
       }
-      bad |= ok && !(isfinite(nx) && isfinite(ny));
+      // (the flag reports the steps' nonlinearity, not a gradient's values)
+      if constexpr (MODEL != kPlaneAdjoint) bad |= ok && !(isfinite(nx) && isfinite(ny));
       v[m] = mk<C>(nx, ny);
     }
     plane_x_forward<Real, C, M>(v, row, tw, j, ok);

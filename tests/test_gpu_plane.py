@@ -118,6 +118,25 @@ def test_adjoint_against_general_path(monkeypatch, n, prec, tol):
     assert abs(n1 - n0) <= tol * max(abs(n0), np.abs(w).sum())
 
 
+@pytest.mark.parametrize("plane", ["1", "0"])
+def test_adjoint_of_a_nonfinite_gradient(monkeypatch, plane):
+    """Infinities in dLoss/dpsi_T come out as what they are: the non-finite flag
+    reports the model's own field, which is finite here."""
+    monkeypatch.setenv("OPFC_PLANE", plane)
+    n = (32, 16, 32)
+    m = ob.PfcB200(n, PI4, r=-0.25, precision=ob.FP64)
+    m.initialize(0.5)
+    m.set_psi(ob.ic_noise(n, -0.285, 0.01, 8))
+    m.forward_checkpointed(3, 2)
+    w = ob.ic_noise(n, 0.0, 1.0, 9)
+    w[1, 2, 3] = np.inf
+    g, _, _ = m.adjoint(w)
+    assert not np.isfinite(g).all()
+    m.step(1)
+    m.sync()
+    assert np.isfinite(m.get_psi()).all()
+
+
 @pytest.mark.parametrize("prec", [ob.FP64, ob.FP32])
 def test_ensemble(oracle, prec):
     sides = [(32, 16, 48), (48, 96, 16), (80, 48, 32), (128, 128, 16), (96, 80, 16), (64, 64, 64)]
