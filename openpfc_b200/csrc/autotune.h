@@ -43,14 +43,15 @@ class AutoTuner {
   }
 
   // time `run(v)` for v in [0, n) on `s`; cache and return the fastest.
-  // `run` returns 0 on success; failing candidates are skipped.
-  int tune(const std::string &key, int n, const std::function<int(int)> &run, cudaStream_t s,
+  // `run` returns 0 on success; failing candidates are skipped.  Without tuning
+  // (or without a candidate that ran) the cached choice or `fallback`, as get_config.
+  int tune(const std::string &key, int n, int fallback, const std::function<int(int)> &run, cudaStream_t s,
            std::vector<double> *ms_out = nullptr) {
     {
       std::lock_guard<std::mutex> lock(mu_);
       refresh();
     }
-    if (disabled_ || mode_ == "fallback_only" || mode_ == "cache_only") return get_config(key, 0);
+    if (disabled_ || mode_ == "fallback_only" || mode_ == "cache_only") return get_config(key, fallback);
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -80,7 +81,7 @@ class AutoTuner {
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (best < 0) return 0;
+    if (best < 0) return fallback;
     std::lock_guard<std::mutex> lock(mu_);
     Table &t = table();
     t.entries[key] = {best, best_ms};

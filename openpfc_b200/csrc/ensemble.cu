@@ -565,13 +565,13 @@ int opfc_ensemble_autotune(opfc_ensemble *e, double *ms_col, double *ms_x, doubl
   ECUDA(e, cudaSetDevice(e->device));
   std::vector<double> mc, mx, mu;
   // the passes run in place on whatever the arrays hold; states are re-set after
-  e->var_col = AutoTuner::instance().tune(e->key + "/col", kVariants,
+  e->var_col = AutoTuner::instance().tune(e->key + "/col", kVariants, 0,
                                           [&](int v) { return launch_stage(e, 2, v); }, e->stream, &mc);
-  e->var_x = AutoTuner::instance().tune(e->key + "/x", kVariants, [&](int v) { return launch_stage(e, 1, v); },
+  e->var_x = AutoTuner::instance().tune(e->key + "/x", kVariants, 0, [&](int v) { return launch_stage(e, 1, v); },
                                         e->stream, &mx);
   // 0: the y, x and y passes, 1: the plane kernel
   e->plane = AutoTuner::instance().tune(
-                 e->key + "/xy", 2,
+                 e->key + "/xy", 2, 1,
                  [&](int v) {
                    if (v == 1) return launch_planes(e);
                    int r = launch_stage(e, 0, e->var_col);
@@ -579,7 +579,7 @@ int opfc_ensemble_autotune(opfc_ensemble *e, double *ms_col, double *ms_x, doubl
                    return r ? r : launch_stage(e, 2, e->var_col);
                  },
                  e->stream) == 1;
-  e->var_upd = AutoTuner::instance().tune(e->key + "/upd", kVariants,
+  e->var_upd = AutoTuner::instance().tune(e->key + "/upd", kVariants, 0,
                                           [&](int v) { return launch_stage(e, 3, v); }, e->stream, &mu);
   ECUDA(e, cudaStreamSynchronize(e->stream));
   cudaMemset(e->flag, 0, sizeof(unsigned));

@@ -1921,13 +1921,13 @@ int opfc_autotune(opfc_handle *h, double *ms) {
   AutoTuner &T = AutoTuner::instance();
   std::vector<double> my, mx, mz;
   // each candidate runs its pass alone, in place on whatever the arrays hold
-  h->var_y = T.tune(tune_key(h, "y"), kVarY, [&](int v) { h->var_y = v; return enqueue_step(h, 0); }, h->stream, &my);
-  h->var_x = T.tune(tune_key(h, "x"), kVarX, [&](int v) { h->var_x = v; return enqueue_step(h, 1); }, h->stream, &mx);
+  h->var_y = T.tune(tune_key(h, "y"), kVarY, default_y(h), [&](int v) { h->var_y = v; return enqueue_step(h, 0); }, h->stream, &my);
+  h->var_x = T.tune(tune_key(h, "x"), kVarX, default_x(h), [&](int v) { h->var_x = v; return enqueue_step(h, 1); }, h->stream, &mx);
   // 0: those two passes as three launches, 1: the plane kernel
   h->plane = false;
   if (plane_ok(h))
     h->plane = T.tune(
-                   tune_key(h, "xy"), 2,
+                   tune_key(h, "xy"), 2, plane_default(h),
                    [&](int v) {
                      if (v == 1) return plane_pass(h);
                      int rc = 0;
@@ -1936,7 +1936,7 @@ int opfc_autotune(opfc_handle *h, double *ms) {
                    },
                    h->stream) == 1;
   h->var_z = T.tune(
-      tune_key(h, "z"), kVarZ,
+      tune_key(h, "z"), kVarZ, default_z(h),
       [&](int v) {
         if (v == 1 && !h->rad_ops) return (int)OPFC_ERR_ARG;
         if (z_computed(v) && (two_field(h->desc.model) || user_ops_model(h->desc.model) || h->slab))

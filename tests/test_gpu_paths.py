@@ -189,3 +189,30 @@ def test_filtered_1024_axes(oracle, path, prec, tol, n):
     m.step(6)
     m.sync()
     assert rel_l2(m.get_psi(), ref) <= tol
+
+
+@pytest.mark.parametrize("off", [("OPENPFC_GPU_AUTOTUNE_DISABLE", "1"), ("OPENPFC_GPU_AUTOTUNE_MODE", "fallback_only"),
+                                 ("OPENPFC_GPU_AUTOTUNE_MODE", "cache_only")])
+@pytest.mark.parametrize("n", [(64, 64, 64), (256, 48, 256), (512, 16, 1024)])
+def test_autotune_without_tuning_keeps_the_defaults(tmp_path, monkeypatch, off, n):
+    """Where tuning is switched off, or only an (empty) cache may be read, autotune()
+    leaves a handle and an ensemble as initialize() made them."""
+    monkeypatch.setenv("OPENPFC_GPU_AUTOTUNE_CACHE_DIR", str(tmp_path))
+    monkeypatch.setenv(*off)
+    m = ob.FilteredB200(n, PI4, precision=ob.FP32)
+    m.initialize(0.5)
+    before = m.variants(), m.kernels_per_step()
+    m.autotune()
+    assert (m.variants(), m.kernels_per_step()) == before
+    psi0 = ob.ic_noise((64, 32, 48), -0.285, 0.01, 3)
+    got = []
+    for tune in (False, True):  # the ensemble's plane kernel rounds differently from its stages
+        e = ob.Ensemble([dict(n=(64, 32, 48), dx=PI4, r=-0.2)], precision=ob.FP32)
+        e.initialize(0.5)
+        if tune:
+            e.autotune()
+        e.set_psi(0, psi0)
+        e.step(5)
+        e.sync()
+        got.append(e.get_psi(0))
+    assert np.array_equal(*got)
