@@ -149,6 +149,13 @@ int launch_stage(opfc_ensemble *e, int stage, int variant) {
                               : ens_launch_stage<float>(stage, W, G, e->num_sms, tiles, e->count, a, e->stream);
 }
 
+// the plane kernel or the separate passes: OPFC_PLANE, else the pick (default,
+// cached or just timed)
+bool plane_choice(bool pick) {
+  const char *pv = std::getenv("OPFC_PLANE");
+  return pv ? std::atoi(pv) == 1 : pick;
+}
+
 int launch_planes(opfc_ensemble *e) {
   const EnsArgs a = args(e, e->d_prefix_plane, e->d_order_plane);
   return e->prec == OPFC_FP64 ? ens_launch_plane<double>(e->planes, e->plane_smem, a, e->stream)
@@ -426,8 +433,7 @@ int opfc_ensemble_create(int count, const opfc_desc *descs, opfc_ensemble **out)
       return bail(OPFC_ERR_CUDA);
     for (cudaEvent_t &v : ep->ev)
       if (cudaEventCreateWithFlags(&v, cudaEventDisableTiming) != cudaSuccess) return bail(OPFC_ERR_CUDA);
-    const char *pv = std::getenv("OPFC_PLANE");
-    ep->plane = !(pv && pv[0] == '0') && AutoTuner::instance().get_config(e->key + "/xy", 1) == 1;
+    ep->plane = plane_choice(AutoTuner::instance().get_config(e->key + "/xy", 1) == 1);
   }
   if (cudaMemset(ep->flag, 0, sizeof(unsigned)) != cudaSuccess || cudaMemset(ep->psi_hat, 0, cb) != cudaSuccess ||
       cudaMemset(ep->work, 0, cb) != cudaSuccess)
@@ -570,15 +576,15 @@ int opfc_ensemble_autotune(opfc_ensemble *e, double *ms_col, double *ms_x, doubl
   e->var_x = AutoTuner::instance().tune(e->key + "/x", kVariants, 0, [&](int v) { return launch_stage(e, 1, v); },
                                         e->stream, &mx);
   // 0: the y, x and y passes, 1: the plane kernel
-  e->plane = AutoTuner::instance().tune(
-                 e->key + "/xy", 2, 1,
-                 [&](int v) {
-                   if (v == 1) return launch_planes(e);
-                   int r = launch_stage(e, 0, e->var_col);
-                   if (!r) r = launch_stage(e, 1, e->var_x);
-                   return r ? r : launch_stage(e, 2, e->var_col);
-                 },
-                 e->stream) == 1;
+  e->plane = plane_choice(AutoTuner::instance().tune(
+                              e->key + "/xy", 2, 1,
+                              [&](int v) {
+                                if (v == 1) return launch_planes(e);
+                                int r = launch_stage(e, 0, e->var_col);
+                                if (!r) r = launch_stage(e, 1, e->var_x);
+                                return r ? r : launch_stage(e, 2, e->var_col);
+                              },
+                              e->stream) == 1);
   e->var_upd = AutoTuner::instance().tune(e->key + "/upd", kVariants, 0,
                                           [&](int v) { return launch_stage(e, 3, v); }, e->stream, &mu);
   ECUDA(e, cudaStreamSynchronize(e->stream));

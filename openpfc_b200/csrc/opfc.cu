@@ -1558,19 +1558,21 @@ int opfc_initialize(opfc_handle *h, double dt) {
   return finish_initialize(h);
 }
 
-// kernel variants and handle state after the operator tables exist
-static int finish_initialize(opfc_handle *h) {
+// The variants that the handle runs: its picks (defaults, cached or just timed),
+// then what the environment forces (OPFC_Y_VARIANT / OPFC_X_VARIANT /
+// OPFC_Z_VARIANT, OPFC_PLANE), then what this handle can run.
+static void settle_variants(opfc_handle *h, int y, int x, int z, bool plane) {
   const int model = h->desc.model;
-  // kernel variants: the autotuner's cached choice, else the defaults;
-  // OPFC_Y_VARIANT / OPFC_X_VARIANT / OPFC_Z_VARIANT force a pass's variant
-  h->var_y = AutoTuner::instance().get_config(tune_key(h, "y"), default_y(h));
-  h->var_x = AutoTuner::instance().get_config(tune_key(h, "x"), default_x(h));
-  h->var_z = AutoTuner::instance().get_config(tune_key(h, "z"), default_z(h));
+  h->var_y = y;
+  h->var_x = x;
+  h->var_z = z;
   // a cached FP32 choice with per-mode FP32 operators needs the opt-in
   if (z_computed(h->var_z) && h->prec == OPFC_FP32 && !computed_ops_allowed()) h->var_z = h->fold_ops ? 6 : 0;
-  if (const char *zv = std::getenv("OPFC_Z_VARIANT")) h->var_z = std::atoi(zv);
-  if (const char *yv = std::getenv("OPFC_Y_VARIANT")) h->var_y = std::atoi(yv);
-  if (const char *xv = std::getenv("OPFC_X_VARIANT")) h->var_x = std::atoi(xv);
+  const char *yv = std::getenv("OPFC_Y_VARIANT"), *xv = std::getenv("OPFC_X_VARIANT"),
+             *zv = std::getenv("OPFC_Z_VARIANT"), *pv = std::getenv("OPFC_PLANE");
+  if (zv) h->var_z = std::atoi(zv);
+  if (yv) h->var_y = std::atoi(yv);
+  if (xv) h->var_x = std::atoi(xv);
   if (h->var_x < 0 || h->var_x >= kVarX) h->var_x = 0;
   if (h->var_z < 0 || h->var_z >= kVarZ) h->var_z = 0;
   if (h->var_z == 1 && !h->rad_ops) h->var_z = 0;
@@ -1578,11 +1580,16 @@ static int finish_initialize(opfc_handle *h) {
     h->var_z = h->var_z == 4 ? 2 : 0;
   if (z_folded(h->var_z) && !h->fold_ops) h->var_z = h->var_z == 7 ? 2 : 0;
   if (h->var_y < 0 || h->var_y >= kVarY) h->var_y = 0;
-  // a forced y or x variant keeps the separate passes
-  const char *pv = std::getenv("OPFC_PLANE");
-  h->plane = AutoTuner::instance().get_config(tune_key(h, "xy"), plane_default(h)) == 1 && plane_ok(h) &&
-             !std::getenv("OPFC_Y_VARIANT") && !std::getenv("OPFC_X_VARIANT");
-  if (pv) h->plane = std::atoi(pv) == 1 && plane_ok(h);
+  // a forced y or x variant and OPFC_NO_TMA name separate passes
+  h->plane = plane_ok(h) && (pv ? std::atoi(pv) == 1 : plane && h->use_tma && !yv && !xv);
+}
+
+// handle state after the operator tables exist
+static int finish_initialize(opfc_handle *h) {
+  AutoTuner &T = AutoTuner::instance();
+  settle_variants(h, T.get_config(tune_key(h, "y"), default_y(h)), T.get_config(tune_key(h, "x"), default_x(h)),
+                  T.get_config(tune_key(h, "z"), default_z(h)),
+                  T.get_config(tune_key(h, "xy"), plane_default(h)) == 1);
   h->initialized = true;
   h->a_valid = false;
   release_graph(h);
@@ -1921,21 +1928,23 @@ int opfc_autotune(opfc_handle *h, double *ms) {
   AutoTuner &T = AutoTuner::instance();
   std::vector<double> my, mx, mz;
   // each candidate runs its pass alone, in place on whatever the arrays hold
-  h->var_y = T.tune(tune_key(h, "y"), kVarY, default_y(h), [&](int v) { h->var_y = v; return enqueue_step(h, 0); }, h->stream, &my);
-  h->var_x = T.tune(tune_key(h, "x"), kVarX, default_x(h), [&](int v) { h->var_x = v; return enqueue_step(h, 1); }, h->stream, &mx);
+  const int y = T.tune(
+      tune_key(h, "y"), kVarY, default_y(h), [&](int v) { h->var_y = v; return enqueue_step(h, 0); }, h->stream, &my);
+  h->var_y = y;
+  const int x = T.tune(
+      tune_key(h, "x"), kVarX, default_x(h), [&](int v) { h->var_x = v; return enqueue_step(h, 1); }, h->stream, &mx);
+  h->var_x = x;
   // 0: those two passes as three launches, 1: the plane kernel
-  h->plane = false;
-  if (plane_ok(h))
-    h->plane = T.tune(
-                   tune_key(h, "xy"), 2, plane_default(h),
-                   [&](int v) {
-                     if (v == 1) return plane_pass(h);
-                     int rc = 0;
-                     for (int k = 0; k < 3 && !rc; ++k) rc = enqueue_step(h, k);
-                     return rc;
-                   },
-                   h->stream) == 1;
-  h->var_z = T.tune(
+  const bool plane = plane_ok(h) && T.tune(
+                                        tune_key(h, "xy"), 2, plane_default(h),
+                                        [&](int v) {
+                                          if (v == 1) return plane_pass(h);
+                                          int rc = 0;
+                                          for (int k = 0; k < 3 && !rc; ++k) rc = enqueue_step(h, k);
+                                          return rc;
+                                        },
+                                        h->stream) == 1;
+  const int z = T.tune(
       tune_key(h, "z"), kVarZ, default_z(h),
       [&](int v) {
         if (v == 1 && !h->rad_ops) return (int)OPFC_ERR_ARG;
@@ -1949,6 +1958,7 @@ int opfc_autotune(opfc_handle *h, double *ms) {
         return enqueue_step(h, 3);
       },
       h->stream, &mz);
+  settle_variants(h, y, x, z, plane);
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   cudaMemset(h->flag, 0, sizeof(unsigned int));
   h->have_state = false;  // the passes overwrote the state

@@ -216,3 +216,34 @@ def test_autotune_without_tuning_keeps_the_defaults(tmp_path, monkeypatch, off, 
         e.sync()
         got.append(e.get_psi(0))
     assert np.array_equal(*got)
+
+
+def test_autotune_keeps_what_the_environment_forces(tmp_path, monkeypatch):
+    """OPFC_PLANE, a forced variant and OPFC_NO_TMA hold after autotune() and against
+    a cached choice (64x64x64 FP32 takes the plane kernel: three kernels a step)."""
+    monkeypatch.setenv("OPENPFC_GPU_AUTOTUNE_CACHE_DIR", str(tmp_path))
+    monkeypatch.delenv("OPENPFC_GPU_AUTOTUNE_MODE", raising=False)
+
+    def kernels(tune, **env):
+        with monkeypatch.context() as c:
+            for k, v in env.items():
+                c.setenv(k, v)
+            m = ob.PfcB200((64, 64, 64), PI4, precision=ob.FP32)
+            m.initialize(0.5)
+            if tune:
+                m.autotune()
+            return m.kernels_per_step(), m.variants()
+
+    for tune in (True, False):  # False: the cached choices
+        assert kernels(tune, OPFC_PLANE="0")[0] == 5
+        assert kernels(tune, OPFC_PLANE="1")[0] == 3
+        assert kernels(tune, OPFC_X_VARIANT="1")[0] == 5
+        assert kernels(tune, OPFC_X_VARIANT="1")[1][1] == 1
+        assert kernels(tune, OPFC_Y_VARIANT="2")[1][0] == 2
+    f = [f for f in tmp_path.iterdir() if f.name.endswith("_opfc_autotune.json")][0]
+    text = f.read_text()
+    assert "/xy/" in text
+    f.write_text("{\n" + "\n".join(line.replace("[0,", "[1,") if "/xy/" in line else line
+                                   for line in text.splitlines()[1:]) + "\n")
+    monkeypatch.setenv("OPENPFC_GPU_AUTOTUNE_CACHE_DIR", str(tmp_path) + "/.")  # read the file again
+    assert kernels(False)[0] == 3 and kernels(False, OPFC_NO_TMA="1")[0] == 5
