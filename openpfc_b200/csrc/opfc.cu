@@ -475,6 +475,10 @@ std::string tune_key(const opfc_handle *h, const char *pass) {
   return b;
 }
 
+// the choice between the y, x and y passes and the plane kernel: an Aluminum step
+// carries three fields with a temperature gradient and two without
+const char *xy_key(const opfc_handle *h) { return h->al_grad ? "xy3" : "xy"; }
+
 // A <- F_z^-1[psi_hat] (and, for TUNGSTEN, B <- F_z^-1[chi psi_hat]); FILTERED
 // keeps only the filtered density in A.
 int prepare_a(opfc_handle *h) {
@@ -1589,7 +1593,7 @@ static int finish_initialize(opfc_handle *h) {
   AutoTuner &T = AutoTuner::instance();
   settle_variants(h, T.get_config(tune_key(h, "y"), default_y(h)), T.get_config(tune_key(h, "x"), default_x(h)),
                   T.get_config(tune_key(h, "z"), default_z(h)),
-                  T.get_config(tune_key(h, "xy"), plane_default(h)) == 1);
+                  T.get_config(tune_key(h, xy_key(h)), plane_default(h)) == 1);
   h->initialized = true;
   h->a_valid = false;
   release_graph(h);
@@ -1936,7 +1940,7 @@ int opfc_autotune(opfc_handle *h, double *ms) {
   h->var_x = x;
   // 0: those two passes as three launches, 1: the plane kernel
   const bool plane = plane_ok(h) && T.tune(
-                                        tune_key(h, "xy"), 2, plane_default(h),
+                                        tune_key(h, xy_key(h)), 2, plane_default(h),
                                         [&](int v) {
                                           if (v == 1) return plane_pass(h);
                                           int rc = 0;

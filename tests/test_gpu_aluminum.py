@@ -86,3 +86,18 @@ def test_aluminum_moving_gradient_vs_oracle(oracle, prec, tol):
     # the gradient acts: without it the result differs
     base = oracle.run_aluminum(psi0, [1.0] * 3, origin, oracle.AluminumParams.test_case(), 1e-2, 4, t0=0.3)
     assert np.abs(ref - base).max() > 1e-6
+
+
+def test_plane_choice_is_cached_by_fields(tmp_path, monkeypatch):
+    """A moving gradient adds a third field to the step: its choice between the
+    passes and the plane kernel is kept apart from the two-field step's."""
+    monkeypatch.setenv("OPENPFC_GPU_AUTOTUNE_CACHE_DIR", str(tmp_path))
+    monkeypatch.delenv("OPENPFC_GPU_AUTOTUNE_MODE", raising=False)
+    for g in (0.0, 2.0):
+        p = params()
+        p.G_grid = g
+        m = ob.AluminumB200((32, 32, 32), [1.0] * 3, p, precision=ob.FP64)
+        m.initialize(1e-2)
+        m.autotune()
+    text = "".join(f.read_text() for f in tmp_path.iterdir())
+    assert "/xy/" in text and "/xy3/" in text
