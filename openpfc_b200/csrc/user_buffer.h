@@ -11,6 +11,9 @@ inline bool own_device_memory(const cudaPointerAttributes &a, int device) {
   return a.type == cudaMemoryTypeDevice && a.device == device;
 }
 
+// page-locked host memory: one asynchronous copy moves it at the link's rate
+inline bool pinned_host_memory(const cudaPointerAttributes &a) { return a.type == cudaMemoryTypeHost; }
+
 // attributes of p; an unregistered host pointer where CUDA does not know it
 inline cudaPointerAttributes pointer_attributes(const void *p) {
   cudaPointerAttributes a{};

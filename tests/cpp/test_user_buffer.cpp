@@ -24,6 +24,10 @@ int main() {
     CHECK(!own_device_memory(at(cudaMemoryTypeManaged, dev), dev));
     CHECK(!own_device_memory(at(cudaMemoryTypeHost, dev), dev));
     CHECK(!own_device_memory(at(cudaMemoryTypeUnregistered, dev), dev));
+    CHECK(pinned_host_memory(at(cudaMemoryTypeHost, dev)));
+    CHECK(!pinned_host_memory(at(cudaMemoryTypeDevice, dev)));
+    CHECK(!pinned_host_memory(at(cudaMemoryTypeManaged, dev)));
+    CHECK(!pinned_host_memory(at(cudaMemoryTypeUnregistered, dev)));
   }
   return bad;
 }

@@ -56,3 +56,33 @@ def test_read_binary_short_file(tmp_path):
         m.read_binary(str(tmp_path / "short.bin"))
     with pytest.raises(ob.OpfcError):
         m.write_binary(str(tmp_path / "bad_%s.bin"))
+
+
+@pytest.mark.parametrize("prec", [ob.FP64, ob.FP32])
+@pytest.mark.parametrize("pinned", [True, False])
+@pytest.mark.parametrize("n", [(32, 16, 24), (128, 96, 128), (256, 256, 128)])
+def test_host_arrays_of_either_precision(prec, pinned, n):
+    """Fields from pinned and pageable host memory, of the handle's precision (one
+    copy where pinned) and of the other one (converted on the way): the same state,
+    and the same values out, as from a device tensor."""
+    import torch
+
+    x = torch.from_numpy(ob.ic_noise(n, -0.285, 0.01, 5)).float().double()  # exact in both precisions
+    own = torch.float64 if prec == ob.FP64 else torch.float32
+    m = ob.PfcB200(n, [1.0] * 3, precision=prec)
+    m.initialize(0.5)
+    m.set_psi(x.to(own).cuda())
+    ref = torch.empty(x.shape, dtype=own, device="cuda")
+    m.get_psi(ref)
+    m.sync()
+    mass = m.mass()
+    for dt in (torch.float64, torch.float32):
+        h = x.to(dt)
+        out = torch.zeros_like(h)
+        if pinned:
+            h, out = h.pin_memory(), out.pin_memory()
+        m.set_psi(h)
+        h.zero_()  # the call has read it
+        assert abs(m.mass() - mass) <= 1e-15
+        m.get_psi(out)
+        assert torch.equal(out, ref.cpu().to(dt))
