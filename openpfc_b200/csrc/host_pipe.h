@@ -54,7 +54,7 @@ class HostPipe {
   cudaError_t in(int device, const H *src, D *dst, size_t n, cudaStream_t s, std::vector<double> *parts) {
     if (std::is_same<H, D>::value && !parts && pinned_host_memory(pointer_attributes(src)))
       return cudaMemcpyAsync(dst, src, n * sizeof(D), cudaMemcpyHostToDevice, s);
-    return run<D>(device, n, parts, [=](size_t lo, size_t hi, D *const *slot, cudaEvent_t *ev, LaneSum *sum) {
+    return run<D>(device, n, s, parts, [=](size_t lo, size_t hi, D *const *slot, cudaEvent_t *ev, LaneSum *sum) {
       constexpr size_t step = kSlotBytes / sizeof(D);
       cudaError_t e = cudaSuccess;
       int k = 0;
@@ -78,7 +78,7 @@ class HostPipe {
       const cudaError_t e = cudaMemcpyAsync(dst, src, n * sizeof(D), cudaMemcpyDeviceToHost, s);
       return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
     }
-    return run<D>(device, n, nullptr, [=](size_t lo, size_t hi, D *const *slot, cudaEvent_t *ev, LaneSum *) {
+    return run<D>(device, n, s, nullptr, [=](size_t lo, size_t hi, D *const *slot, cudaEvent_t *ev, LaneSum *) {
       constexpr size_t step = kSlotBytes / sizeof(D);
       cudaError_t e = cudaSuccess;
       auto issue = [&](size_t i, int k) {
@@ -147,11 +147,15 @@ class HostPipe {
     return cudaSuccess;
   }
 
-  // f(lo, hi, slots, events, sum) on each thread's share of n values of D
-  template <typename D, typename F> cudaError_t run(int device, size_t n, std::vector<double> *parts, const F &f) {
+  // f(lo, hi, slots, events, sum) on each thread's share of n values of D.  The
+  // per-thread default stream is another stream on every thread: the caller's own
+  // thread then does it all.
+  template <typename D, typename F>
+  cudaError_t run(int device, size_t n, cudaStream_t s, std::vector<double> *parts, const F &f) {
     const size_t slots = (n * sizeof(D) + kSlotBytes - 1) / kSlotBytes;
     const size_t cores = std::max(1u, std::thread::hardware_concurrency());
     int T = (int)std::min<size_t>({(size_t)kMaxThreads, cores, std::max<size_t>(1, slots)});
+    if (s == cudaStreamPerThread) T = 1;
     cudaError_t e = ensure(T);
     if (e != cudaSuccess) return e;
     const size_t share = ((n + T - 1) / T + 3) / 4 * 4;

@@ -86,3 +86,19 @@ def test_host_arrays_of_either_precision(prec, pinned, n):
         assert abs(m.mass() - mass) <= 1e-15
         m.get_psi(out)
         assert torch.equal(out, ref.cpu().to(dt))
+
+
+def test_host_arrays_on_the_per_thread_default_stream(oracle):
+    """The per-thread default stream is another stream on every host thread, so the
+    threads that convert a large array must not queue their copies on it."""
+    n = (256, 128, 128)
+    psi0 = ob.ic_noise(n, -0.285, 0.01, 5)
+    m = ob.PfcB200(n, PI4, precision=ob.FP32, stream=2)  # cudaStreamPerThread
+    m.initialize(0.5)
+    ref = None
+    for _ in range(4):
+        m.set_psi(psi0)
+        out = m.get_psi()
+        assert np.abs(out - psi0).max() <= 1e-6
+        ref = out if ref is None else ref
+        assert np.array_equal(out, ref)
