@@ -19,7 +19,6 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <system_error>
 #include <thread>
 #include <type_traits>
 #include <vector>
@@ -173,7 +172,7 @@ class HostPipe {
     int started = 1;  // share 0 runs here
     try {
       for (; started < T; ++started) th.emplace_back(work, started);
-    } catch (const std::system_error &) {  // no more threads: the rest runs here too
+    } catch (...) {  // no more threads (or no memory for one): the rest runs here too
     }
     work(0);
     for (int t = started; t < T; ++t) work(t);
