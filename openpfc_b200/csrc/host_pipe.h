@@ -40,10 +40,17 @@ struct LaneSum {
 
 class HostPipe {
  public:
-  static constexpr size_t kSlotBytes = size_t(1) << 20;
+  static constexpr size_t kShareBytes = size_t(1) << 20;  // device bytes that are worth a thread
+  static constexpr size_t kMinSlot = size_t(1) << 18, kMaxSlot = size_t(1) << 20;
+  static constexpr size_t kOneCopy = size_t(1) << 26;
   static constexpr int kMaxThreads = 16;
 
   ~HostPipe() { release(); }
+
+  // slots for arrays of up to `bytes` device bytes from the first one on: an
+  // ensemble's members come in any order, and slots pinned again as they grow are
+  // paid for each time (setting 64 members: 50 ms so, 36 with one set of slots)
+  void expect(size_t bytes) { expect_ = bytes; }
 
   // n values host (H) -> device (D) on stream s; with `parts`, the compensated
   // sums of the host values are appended to it.  Returns before the last copies
@@ -51,10 +58,10 @@ class HostPipe {
   // that goes as one copy has to stay as it is until then).
   template <typename H, typename D>
   cudaError_t in(int device, const H *src, D *dst, size_t n, cudaStream_t s, std::vector<double> *parts) {
-    if (std::is_same<H, D>::value && !parts && pinned_host_memory(pointer_attributes(src)))
+    if (std::is_same<H, D>::value && !parts && one_copy(src, n * sizeof(D)))
       return cudaMemcpyAsync(dst, src, n * sizeof(D), cudaMemcpyHostToDevice, s);
     return run<D>(device, n, s, parts, [=](size_t lo, size_t hi, D *const *slot, cudaEvent_t *ev, LaneSum *sum) {
-      constexpr size_t step = kSlotBytes / sizeof(D);
+      const size_t step = slot_ / sizeof(D);
       cudaError_t e = cudaSuccess;
       int k = 0;
       for (size_t i = lo; i < hi && e == cudaSuccess; i += step, k ^= 1) {
@@ -73,12 +80,12 @@ class HostPipe {
   // n values device (D) -> host (H), complete on return
   template <typename D, typename H>
   cudaError_t out(int device, const D *src, H *dst, size_t n, cudaStream_t s) {
-    if (std::is_same<H, D>::value && pinned_host_memory(pointer_attributes(dst))) {
+    if (std::is_same<H, D>::value && one_copy(dst, n * sizeof(D))) {
       const cudaError_t e = cudaMemcpyAsync(dst, src, n * sizeof(D), cudaMemcpyDeviceToHost, s);
       return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
     }
     return run<D>(device, n, s, nullptr, [=](size_t lo, size_t hi, D *const *slot, cudaEvent_t *ev, LaneSum *) {
-      constexpr size_t step = kSlotBytes / sizeof(D);
+      const size_t step = slot_ / sizeof(D);
       cudaError_t e = cudaSuccess;
       auto issue = [&](size_t i, int k) {
         if (i >= hi || e != cudaSuccess) return;
@@ -108,13 +115,18 @@ class HostPipe {
     else
       std::free(pin_);
     pin_ = nullptr;
+    pinned_ = tried_pin_ = false;
     threads_ = 0;
+    slot_ = 0;
   }
 
  private:
   char *pin_ = nullptr;
+  bool tried_pin_ = false;  // the slots are pinned, or pinning was refused
   bool pinned_ = false;  // else pageable: the copies are then slower and synchronous, with the same result
   int threads_ = 0;  // threads with slots and events
+  size_t slot_ = 0;  // bytes of a slot
+  size_t expect_ = 0;
   std::vector<cudaEvent_t> ev_;
 
   template <typename A, typename B> static void convert(const A *a, B *b, size_t n) {
@@ -124,16 +136,39 @@ class HostPipe {
       for (size_t i = 0; i < n; ++i) b[i] = (B)a[i];
   }
 
-  cudaError_t ensure(int threads) {
-    if (threads <= threads_) return cudaSuccess;
+  // An array without conversion that no staging would speed up: pinned, or no
+  // larger than kOneCopy (64 MiB: 5.4 to 6.3 ms in as one copy, 4.0 to 4.3 through
+  // slots that cost 5 ms to pin; 512 MiB: 50 and 15).
+  static bool one_copy(const void *host, size_t bytes) {
+    return bytes <= kOneCopy || pinned_host_memory(pointer_attributes(host));
+  }
+
+  static int threads_for(size_t bytes) {
+    const size_t cores = std::max(1u, std::thread::hardware_concurrency());
+    return (int)std::min<size_t>({(size_t)kMaxThreads, cores, std::max<size_t>(1, (bytes + kShareBytes - 1) / kShareBytes)});
+  }
+
+  // Slots and events for arrays of `bytes`.  Pinning costs 0.6 ms a MiB, once: a
+  // slot holds a sixteenth of a thread's share (256 KiB to 1 MiB), and an array of
+  // one share goes through ordinary memory (256 KiB of FP32 from FP64: 0.08 ms
+  // either way, but 1.5 ms for the first call with pinned slots).
+  cudaError_t ensure(size_t bytes) {
+    bytes = std::max(bytes, expect_);
+    const int threads = threads_for(bytes);
+    const bool pin = bytes > kShareBytes;
+    const size_t slot = pin ? std::min(kMaxSlot, std::max(kMinSlot, (bytes / threads / 16 + 4095) / 4096 * 4096)) : kMaxSlot;
+    if (threads <= threads_ && (!pin || (tried_pin_ && slot <= slot_))) return cudaSuccess;
     for (cudaEvent_t e : ev_) cudaEventSynchronize(e);  // copies out of the old slots
     release();
-    cudaError_t e = cudaHostAlloc((void **)&pin_, 2 * kSlotBytes * threads, cudaHostAllocDefault);
-    pinned_ = e == cudaSuccess;
-    if (!pinned_) {
-      cudaGetLastError();
-      if (!(pin_ = static_cast<char *>(std::malloc(2 * kSlotBytes * threads)))) return e;
+    cudaError_t e = cudaSuccess;
+    if (pin) {
+      e = cudaHostAlloc((void **)&pin_, 2 * slot * threads, cudaHostAllocDefault);
+      if (e != cudaSuccess) cudaGetLastError();
+      tried_pin_ = true;
     }
+    pinned_ = pin && e == cudaSuccess;
+    if (!pinned_ && !(pin_ = static_cast<char *>(std::malloc(2 * slot * threads)))) return cudaErrorMemoryAllocation;
+    slot_ = slot;
     for (int i = 0; i < 2 * threads; ++i) {
       cudaEvent_t v = nullptr;
       if ((e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming)) != cudaSuccess) {
@@ -151,19 +186,15 @@ class HostPipe {
   // thread then does it all.
   template <typename D, typename F>
   cudaError_t run(int device, size_t n, cudaStream_t s, std::vector<double> *parts, const F &f) {
-    const size_t slots = (n * sizeof(D) + kSlotBytes - 1) / kSlotBytes;
-    const size_t cores = std::max(1u, std::thread::hardware_concurrency());
-    int T = (int)std::min<size_t>({(size_t)kMaxThreads, cores, std::max<size_t>(1, slots)});
-    if (s == cudaStreamPerThread) T = 1;
-    cudaError_t e = ensure(T);
+    const int T = s == cudaStreamPerThread ? 1 : threads_for(n * sizeof(D));
+    cudaError_t e = ensure(n * sizeof(D));
     if (e != cudaSuccess) return e;
     const size_t share = ((n + T - 1) / T + 3) / 4 * 4;
     std::vector<cudaError_t> rc(T, cudaSuccess);
     std::vector<LaneSum> sums(parts ? T : 0);
     auto work = [&](int t) {
       const size_t lo = std::min(n, share * t), hi = std::min(n, lo + share);
-      D *slot[2] = {reinterpret_cast<D *>(pin_ + 2 * t * kSlotBytes),
-                    reinterpret_cast<D *>(pin_ + (2 * t + 1) * kSlotBytes)};
+      D *slot[2] = {reinterpret_cast<D *>(pin_ + 2 * t * slot_), reinterpret_cast<D *>(pin_ + (2 * t + 1) * slot_)};
       rc[t] = cudaSetDevice(device);
       if (rc[t] == cudaSuccess) rc[t] = f(lo, hi, slot, &ev_[2 * t], parts ? &sums[t] : nullptr);
     };

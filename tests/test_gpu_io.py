@@ -77,7 +77,7 @@ def test_host_arrays_of_either_precision(prec, pinned, n):
     m.sync()
     mass = m.mass()
     for dt in (torch.float64, torch.float32):
-        h = x.to(dt)
+        h = x.to(dt, copy=True)
         out = torch.zeros_like(h)
         if pinned:
             h, out = h.pin_memory(), out.pin_memory()
