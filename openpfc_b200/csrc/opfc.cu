@@ -792,7 +792,7 @@ int ensure_side(opfc_handle *h) {
 // time, which the x pass reads.
 int enqueue_steps(opfc_handle *h, int n) {
   int rc;
-  if (h->al_grad) {
+  if (h->al_grad || n == 1) {  // (one step has no next one to run beside)
     for (int s = 0; s < n; ++s)
       if ((rc = enqueue_step_kernels(h, -1))) return rc;
     return OPFC_OK;
@@ -1703,9 +1703,10 @@ int opfc_step(opfc_handle *h, int n_steps) {
     }
     return OPFC_OK;
   }
-  if ((rc = ensure_side(h))) return rc;
   // From 2^21 cells on the separate passes are long enough to hide their launches.
-  if (!keeps_graph(h) && h->nr >= ((size_t)1 << 21)) return enqueue_steps(h, n_steps);
+  const bool eager = !keeps_graph(h) && h->nr >= ((size_t)1 << 21);
+  if ((eager ? n_steps > 1 : keeps_graph(h) && n_steps >= kGraphSteps) && (rc = ensure_side(h))) return rc;
+  if (eager) return enqueue_steps(h, n_steps);
   while (n_steps > 0) {
     const bool many = keeps_graph(h) && n_steps >= kGraphSteps;
     cudaGraphExec_t *g = many ? &h->graph_many : &h->graph_exec;
