@@ -212,7 +212,9 @@ int opfc_kernels_per_step(const opfc_handle *h);
 /* Measurement hook (no reference counterpart; the reference times FFT calls
  * with MPI_Wtime, fft_heffte_backend.hpp:158-164): times each kernel of the
  * step alone, `reps` launches each, with CUDA events on the handle's stream;
- * ms[k] = mean milliseconds per launch.  Returns the number of kernels timed
+ * ms[k] = mean milliseconds per launch, -1 for a kernel that this handle's step
+ * does not launch (where the y and x passes are one plane kernel, its time is
+ * that of x_fused and the y passes have none).  Returns the number of entries
  * (>= 0) or an error.  The repeated in-place passes leave the field undefined:
  * call opfc_set_psi before stepping again. */
 int opfc_profile_step(opfc_handle *h, int reps, double *ms, int max_kernels);
@@ -221,7 +223,8 @@ const char *opfc_step_kernel_name(int k);
 /* NVTX range name of kernel k: the reference's profiling regions whose work the
  * kernel does (OPENPFC_PROFILE "gradient/mean_field/...", "gradient/evolve/...",
  * apps/tungsten/include/tungsten/cpu/tungsten_model.hpp:313-362), pass in
- * brackets.  opfc_profile_step times each kernel inside its range; with
+ * brackets (a plane kernel runs in x_fused's).  opfc_profile_step times each kernel
+ * inside its range; with
  * OPFC_NVTX=1 in the environment at opfc_create, opfc_step runs eagerly (no
  * CUDA graph) and encloses every kernel in its range and every step in "step",
  * so an NVTX-aware profiler groups the work by the reference's regions. */

@@ -262,13 +262,14 @@ class _ModelBase(_Handle):
         return tuple(v)
 
     def profile_step(self, reps: int = 10) -> dict:
-        """Mean ms per launch of each kernel of the step, timed alone with CUDA
-        events on the handle's stream.  Leaves the field undefined."""
+        """Mean ms per launch of each kernel that the step launches, timed alone with
+        CUDA events on the handle's stream (the plane kernel, in place of the y and x
+        passes, under x_fused).  Leaves the field undefined."""
         ms = (ctypes.c_double * 8)()
         n = lib().opfc_profile_step(self._h, int(reps), ms, 8)
         if n < 0:
             _check(self._h, n)
-        return {lib().opfc_step_kernel_name(k).decode(): ms[k] for k in range(n)}
+        return {lib().opfc_step_kernel_name(k).decode(): ms[k] for k in range(n) if ms[k] >= 0}
 
 
 def _geom(d: Desc, n, dx, origin, precision, device, stream):

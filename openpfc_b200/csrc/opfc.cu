@@ -537,6 +537,10 @@ struct NvtxRange {
 
 int enqueue_step_kernels(opfc_handle *h, int only);
 
+// What the step launches in place of kernel k: where the y and x passes are one
+// plane kernel, that one for x_fused and nothing (-1) for the y passes.
+int launched_as(const opfc_handle *h, int k) { return !h->plane || k > 2 ? k : k == 1 ? kStepXY : -1; }
+
 // Enqueue the step's kernels on h->stream; `only` >= 0 enqueues that one
 // kernel.  With NVTX ranges on (eager steps, opfc_profile_step) each kernel is
 // enqueued inside the range of its reference region.
@@ -544,8 +548,10 @@ int enqueue_step(opfc_handle *h, int only = -1) {
   if (!h->nvtx) return enqueue_step_kernels(h, only);
   for (int k = 0; k < kStepKernels; ++k) {
     if (only >= 0 && k != only) continue;
+    const int launch = only >= 0 ? only : launched_as(h, k);
+    if (launch < 0) continue;
     NvtxRange range(kStepRegions[k]);
-    const int rc = enqueue_step_kernels(h, k);
+    const int rc = enqueue_step_kernels(h, launch);
     if (rc) return rc;
   }
   return OPFC_OK;
@@ -1999,10 +2005,13 @@ int opfc_profile_step(opfc_handle *h, int reps, double *ms, int max_kernels) {
   for (int k = 0; k < nk; ++k) {
     // one untimed launch, then `reps` timed launches of kernel k alone, inside
     // the NVTX range of its reference region
+    const int launch = launched_as(h, k);
+    ms[k] = -1.0;
+    if (launch < 0) continue;
     NvtxRange range(kStepRegions[k]);
-    if ((rc = enqueue_step_kernels(h, k))) break;
+    if ((rc = enqueue_step_kernels(h, launch))) break;
     cudaEventRecord(e0, h->stream);
-    for (int r = 0; r < reps && !rc; ++r) rc = enqueue_step_kernels(h, k);
+    for (int r = 0; r < reps && !rc; ++r) rc = enqueue_step_kernels(h, launch);
     cudaEventRecord(e1, h->stream);
     cudaEventSynchronize(e1);
     float t = 0;

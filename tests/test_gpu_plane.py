@@ -119,6 +119,27 @@ def test_adjoint_against_general_path(monkeypatch, n, prec, tol):
 
 
 @pytest.mark.parametrize("plane", ["1", "0"])
+def test_profile_and_nvtx_run_the_steps_kernels(monkeypatch, plane):
+    """opfc_profile_step times what the step launches, and steps with NVTX ranges are
+    the same steps (the plane kernel rounds differently from the passes)."""
+    monkeypatch.setenv("OPFC_PLANE", plane)
+    n = (64, 64, 48)
+    psi0 = ob.ic_noise(n, -0.285, 0.01, 8)
+    got = []
+    for nvtx in ("0", "1"):
+        monkeypatch.setenv("OPFC_NVTX", nvtx)
+        m = ob.PfcB200(n, PI4, r=-0.25, precision=ob.FP32)
+        m.initialize(0.5)
+        m.set_psi(psi0)
+        m.step(12)
+        m.sync()
+        got.append(m.get_psi())
+    assert np.array_equal(*got)
+    y = set() if plane == "1" else {"y_inverse", "y_forward"}
+    assert set(m.profile_step(2)) == {"x_fused", "z_update", "hermitian_fix"} | y
+
+
+@pytest.mark.parametrize("plane", ["1", "0"])
 def test_adjoint_of_a_nonfinite_gradient(monkeypatch, plane):
     """Infinities in dLoss/dpsi_T come out as what they are: the non-finite flag
     reports the model's own field, which is finite here."""
