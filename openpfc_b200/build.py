@@ -25,7 +25,7 @@ SOURCES = ["kernels_f32.cu", "kernels_f64.cu", "ensemble_f32.cu", "ensemble_f64.
            "ens_plane_f64.cu", "aluminum_f32.cu", "aluminum_f64.cu", "opfc.cu", "noalloc.cu",
            "ensemble.cu", "io.cu", "wait_check.cu"]
 HEADERS = ["fft_core.cuh", "kernels.cuh", "launch.h", "col_tma.cuh", "x_tma.cuh", "x_sq.cuh", "twiddle.h",
-           "ensemble.cuh", "autotune.h", "io.h", "plane.cuh", "plane.h", "host_pipe.h", "user_buffer.h", "ens_plane.cuh", "aluminum.cuh"]
+           "ensemble.cuh", "autotune.h", "io.h", "plane.cuh", "plane.h", "host_pipe.h", "user_buffer.h", "recent_table.h", "ens_plane.cuh", "aluminum.cuh"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",

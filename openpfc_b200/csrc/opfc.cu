@@ -21,6 +21,7 @@
 #include <random>
 #include <string>
 #include <thread>
+#include <tuple>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -30,6 +31,7 @@
 #include "host_pipe.h"
 #include "launch.h"
 #include "plane.h"
+#include "recent_table.h"
 #include "twiddle.h"
 #include "user_buffer.h"
 #include "autotune.h"
@@ -201,12 +203,9 @@ struct opfc_handle {
   // the transform's own x and y passes as one plane kernel
   bool plane_fft = false;
   int num_sms = 148;
-  struct Tmap {
-    const void *ptr;
-    int axis, W, real;
-    CUtensorMap map;
-  };
-  std::vector<Tmap> tmaps;
+  // tensor maps by (array, axis, W, real); a launch uses at most five and copies
+  // them, a long segment of the adjoint has more arrays than places
+  RecentTable<std::tuple<const void *, int, int, int>, CUtensorMap, 64> tmaps;
   std::string err;
 };
 
@@ -385,11 +384,10 @@ int col_plain(opfc_handle *h, int axis, int dir, const void *in0, void *out0,
 
 const CUtensorMap *tmap_for(opfc_handle *h, const void *ptr, int axis, int W, bool real) {
   if (!ptr) return nullptr;
-  for (const auto &t : h->tmaps)
-    if (t.ptr == ptr && t.axis == axis && t.W == W && t.real == (int)real) return &t.map;
+  const auto key = std::make_tuple(ptr, axis, W, (int)real);
+  if (const CUtensorMap *m = h->tmaps.find(key)) return m;
   EncodeTiledFn enc = encode_fn();
-  // returned pointers must stay valid while a launch is assembled: never grow
-  if (!enc || h->tmaps.size() == h->tmaps.capacity()) return nullptr;
+  if (!enc) return nullptr;
   const cuuint64_t es = h->rsz, S = real ? 1 : 2;
   const int N = axis == 1 ? h->n1 : h->n2;
   const cuuint32_t RB = (cuuint32_t)std::min(N, 256);
@@ -397,12 +395,8 @@ const CUtensorMap *tmap_for(opfc_handle *h, const void *ptr, int axis, int W, bo
   cuuint64_t strides[2] = {S * h->M * es, S * h->M * (cuuint64_t)h->n1 * es};
   cuuint32_t box[3] = {(cuuint32_t)(S * W), axis == 1 ? RB : 1u, axis == 1 ? 1u : RB};
   cuuint32_t estr[3] = {1, 1, 1};
-  opfc_handle::Tmap t{};
-  t.ptr = ptr;
-  t.axis = axis;
-  t.W = W;
-  t.real = (int)real;
-  const CUresult r = enc(&t.map, es == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
+  CUtensorMap map;
+  const CUresult r = enc(&map, es == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
                          3, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                          CU_TENSOR_MAP_SWIZZLE_NONE,
                          // full 128-byte rows may pull in the neighbouring tile's
@@ -411,9 +405,7 @@ const CUtensorMap *tmap_for(opfc_handle *h, const void *ptr, int axis, int W, bo
                          S * W * es >= 128 ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B
                                            : CU_TENSOR_MAP_L2_PROMOTION_NONE,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return nullptr;
-  h->tmaps.push_back(t);
-  return &h->tmaps.back().map;
+  return r == CUDA_SUCCESS ? h->tmaps.keep(key, map) : nullptr;
 }
 
 // Tensor map of a folded table ((M+1) x (N1/2+1) x (N2/2+1) modes in the split
@@ -422,28 +414,22 @@ const CUtensorMap *tmap_for(opfc_handle *h, const void *ptr, int axis, int W, bo
 const CUtensorMap *tmap_fold(opfc_handle *h, const void *ptr, int W, bool pairs) {
   if (!ptr || h->n2 % 16 != 0) return nullptr;
   const int axis = pairs ? 3 : 4;  // cache keys apart from the full arrays' maps
-  for (const auto &t : h->tmaps)
-    if (t.ptr == ptr && t.axis == axis && t.W == W) return &t.map;
+  const auto key = std::make_tuple(ptr, axis, W, pairs ? 0 : 1);
+  if (const CUtensorMap *m = h->tmaps.find(key)) return m;
   EncodeTiledFn enc = encode_fn();
-  if (!enc || h->tmaps.size() == h->tmaps.capacity()) return nullptr;
+  if (!enc) return nullptr;
   const cuuint64_t es = h->rsz, S = pairs ? 2 : 1;
   const cuuint64_t F1 = h->n1 / 2 + 1, F2 = h->n2 / 2 + 1;
   cuuint64_t dims[3] = {S * (cuuint64_t)h->M, F1, F2};
   cuuint64_t strides[2] = {S * h->M * es, S * h->M * F1 * es};
   cuuint32_t box[3] = {(cuuint32_t)(S * W), 1u, (cuuint32_t)(h->n2 / 4)};
   cuuint32_t estr[3] = {1, 1, 1};
-  opfc_handle::Tmap t{};
-  t.ptr = ptr;
-  t.axis = axis;
-  t.W = W;
-  t.real = pairs ? 0 : 1;
-  const CUresult r = enc(&t.map, es == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
+  CUtensorMap map;
+  const CUresult r = enc(&map, es == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
                          3, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return nullptr;
-  h->tmaps.push_back(t);
-  return &h->tmaps.back().map;
+  return r == CUDA_SUCCESS ? h->tmaps.keep(key, map) : nullptr;
 }
 
 XLaunch x_base(opfc_handle *h) {
@@ -1336,7 +1322,6 @@ int opfc_create(const opfc_desc *d, opfc_handle **out) {
   if (cudaMemset(hp->psi_hat, 0, cb) != cudaSuccess) return cleanup(OPFC_ERR_CUDA);
   if (cudaDeviceGetAttribute(&hp->num_sms, cudaDevAttrMultiProcessorCount, hp->device) != cudaSuccess)
     hp->num_sms = 148;
-  hp->tmaps.reserve(64);
   hp->plane_fft = plane_fft_default(hp);
   *out = h.release();
   return OPFC_OK;
