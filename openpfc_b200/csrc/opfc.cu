@@ -2445,6 +2445,15 @@ bool adj_plane(const opfc_handle *h) {
 
 int adjoint_buffers(opfc_handle *h) {
   int rc;
+  // The plane kernel's reverse step keeps two more arrays for each step of a
+  // segment.  The program's other allocations come first: it is taken only where
+  // they are no more than a quarter of the memory that is free.
+  const size_t missing_steps = std::max(0, h->ckpt_K - (int)std::min(h->seg_a.size(), h->seg_n.size()));
+  if (adj_plane(h) && missing_steps > 0) {
+    size_t free_b = 0, total = 0;
+    CUDA_TRY(h, cudaMemGetInfo(&free_b, &total));
+    if (missing_steps * 2 * h->nc * 2 * h->rsz > free_b / 4) h->no_adj_plane = true;
+  }
   const bool plane = adj_plane(h);
   for (auto &p : h->adj_c)
     if (!p && (rc = dev_alloc(h, &p, h->nc * 2 * h->rsz))) return rc;
@@ -2645,6 +2654,7 @@ int opfc_adjoint(opfc_handle *h, const void *grad_psi_T, int dtype, int where, v
   if (!h->initialized) return fail(h, OPFC_ERR_STATE, "opfc_adjoint needs the operator tables");
   CUDA_TRY(h, cudaSetDevice(h->device));
   if ((rc = adjoint_tables(h))) return rc;  // r or dt may have changed since the last call
+  h->no_adj_plane = false;
   if ((rc = adjoint_buffers(h))) return rc;
   // lambda_T = dLoss/dpsi_T
   if ((rc = real_in(h, grad_psi_T, dtype, where))) return rc;

@@ -124,3 +124,33 @@ def test_set_r_after_a_failed_rebuild(oracle):
     m.sync()
     ref = oracle.run_plain(psi0, PI4, -0.3, DT, 5)
     assert np.linalg.norm((m.get_psi() - ref).ravel()) <= 1e-11 * np.linalg.norm(ref.ravel())
+
+
+def test_long_segments_leave_memory_to_the_program():
+    """The reverse step that keeps three arrays per step of a segment is taken only
+    where the two additional ones are a small part of the free memory: with 8 GB
+    left, segments of 300 steps keep one."""
+    import torch
+
+    n, K = (32, 16, 1024), 300
+    array = 17 * 16 * 1024 * 16
+    psi0 = ob.ic_noise(n, -0.285, 0.01, 6)
+    w = psi0 - psi0.mean()
+    got = []
+    for full in (False, True):
+        free = torch.cuda.mem_get_info()[0]
+        if free < 16e9:
+            pytest.skip("another program holds this GPU's memory")
+        filler = torch.empty(int(free - 8e9), dtype=torch.uint8, device="cuda") if full else None
+        m = ob.PfcB200(n, PI4, r=-0.25, precision=ob.FP64)
+        m.initialize(DT)
+        m.set_psi(psi0)
+        m.forward_checkpointed(4, K)
+        before = m.get_allocated_memory_bytes()
+        got.append(m.adjoint(w))
+        arrays = (m.get_allocated_memory_bytes() - before) / array
+        assert arrays < 1.2 * K if full else arrays > 2.9 * K, arrays
+        m.close()
+        del filler
+        torch.cuda.empty_cache()
+    assert np.linalg.norm(got[0][0] - got[1][0]) <= 1e-10 * np.linalg.norm(got[1][0])
