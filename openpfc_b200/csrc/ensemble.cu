@@ -149,6 +149,28 @@ int launch_stage(opfc_ensemble *e, int stage, int variant) {
                               : ens_launch_stage<float>(stage, W, G, e->num_sms, tiles, e->count, a, e->stream);
 }
 
+// Whether the plane kernel pays when neither the autotuner nor the environment
+// chose.  It saves launches (few cells) and sweeps through HBM (arrays well past
+// the L2); in between it wins on 8 values a thread only, the lengths 64 and 128.
+// One kernel holds the registers of the longest line for all members: 20 and 24
+// values a thread for 80 and 96 points, with spills in FP64.  Separate passes /
+// plane kernel, us a step, FP32: 2 cubes of 32 19.7 / 12.6, 6 of mixed sides (0.73 M
+// cells) 34.4 / 28.3, 64 of 64 248 / 214, 64 of 80 619 / 570, 128 mixed (43 M) 831 /
+// 789; but 64 of 32 63.5 / 66.6, 64 of 48 166 / 184, 8 of 96 128 / 139, 40 mixed (14 M)
+// 286 / 314, 64 mixed (20 M) 407 / 412.  FP64: 4 mixed 65 / 76, 64 mixed 702 / 806, 256
+// mixed 2830 / 3420.
+bool plane_pays(const opfc_ensemble *e) {
+  if (e->prec == OPFC_FP64) return false;
+  double cells = 0, short_lines = 0;
+  for (const EnsInst &in : e->inst) {
+    const double c = (double)in.n0 * in.n1 * in.n2;
+    const bool pow2 = (in.M & (in.M - 1)) == 0 && (in.n1 & (in.n1 - 1)) == 0;
+    cells += c;
+    if (pow2 && in.M * in.n1 >= 32 * 64) short_lines += c;
+  }
+  return cells < 1.3e6 || cells >= 25e6 || short_lines >= 0.5 * cells;
+}
+
 // the plane kernel or the separate passes: OPFC_PLANE, else the pick (default,
 // cached or just timed)
 bool plane_choice(bool pick) {
@@ -433,7 +455,7 @@ int opfc_ensemble_create(int count, const opfc_desc *descs, opfc_ensemble **out)
       return bail(OPFC_ERR_CUDA);
     for (cudaEvent_t &v : ep->ev)
       if (cudaEventCreateWithFlags(&v, cudaEventDisableTiming) != cudaSuccess) return bail(OPFC_ERR_CUDA);
-    ep->plane = plane_choice(AutoTuner::instance().get_config(e->key + "/xy", 1) == 1);
+    ep->plane = plane_choice(AutoTuner::instance().get_config(e->key + "/xy", plane_pays(ep)) == 1);
   }
   ep->pipe.expect(ep->nr_max * ep->rsz);
   if (cudaMemset(ep->flag, 0, sizeof(unsigned)) != cudaSuccess || cudaMemset(ep->psi_hat, 0, cb) != cudaSuccess ||
@@ -578,7 +600,7 @@ int opfc_ensemble_autotune(opfc_ensemble *e, double *ms_col, double *ms_x, doubl
                                         e->stream, &mx);
   // 0: the y, x and y passes, 1: the plane kernel
   e->plane = plane_choice(AutoTuner::instance().tune(
-                              e->key + "/xy", 2, 1,
+                              e->key + "/xy", 2, plane_pays(e),
                               [&](int v) {
                                 if (v == 1) return launch_planes(e);
                                 int r = launch_stage(e, 0, e->var_col);

@@ -65,3 +65,25 @@ def test_ensemble_autotune_keeps_results(oracle, tmp_path, monkeypatch):
     for i, m in enumerate(ms):
         ref = oracle.run_plain(psi0[i], PI4, m["r"], 0.5, 5)
         assert rel_l2(e.get_psi(i), ref) <= 1e-5
+
+
+@pytest.mark.parametrize("prec,sides,plane", [(ob.FP32, [32, 48], "1"), (ob.FP32, [64] * 6, "1"),
+                                              (ob.FP32, [96, 96, 80], "0"), (ob.FP64, [32, 48], "0"),
+                                              (ob.FP64, [64] * 6, "0")])
+def test_default_choice_of_the_passes(monkeypatch, prec, sides, plane):
+    """The plane kernel where it was measured to win (few cells, lengths of 64 and
+    128, FP32), the separate passes elsewhere and in FP64; the two round differently."""
+    monkeypatch.setenv("OPENPFC_GPU_AUTOTUNE_MODE", "fallback_only")
+    got = []
+    for force in (None, plane):
+        monkeypatch.delenv("OPFC_PLANE", raising=False)
+        if force:
+            monkeypatch.setenv("OPFC_PLANE", force)
+        e = ob.Ensemble([{"n": (s, s, s), "dx": PI4, "r": -0.25} for s in sides], precision=prec)
+        e.initialize(0.5)
+        for i, s in enumerate(sides):
+            e.set_psi(i, ob.ic_noise((s, s, s), -0.285, 0.01, i))
+        e.step(4)
+        e.sync()
+        got.append([e.get_psi(i) for i in range(len(sides))])
+    assert all(np.array_equal(a, b) for a, b in zip(*got))
