@@ -172,6 +172,7 @@ struct opfc_handle {
   void *adj_r[4] = {nullptr, nullptr, nullptr, nullptr};
 
   cudaGraphExec_t graph_exec = nullptr, graph_many = nullptr;  // one step, kGraphSteps steps
+  int eager_steps = 0;  // steps launched directly since the graphs were released
   cudaStream_t side = nullptr;  // Hermitian projection beside the next step's passes
   cudaEvent_t ev[2] = {nullptr, nullptr};
   HostPipe pipe;  // host arrays in and out
@@ -767,6 +768,7 @@ void release_graph(opfc_handle *h) {
     if (*g) cudaGraphExecDestroy(*g);
     *g = nullptr;
   }
+  h->eager_steps = 0;
 }
 
 // second stream of enqueue_steps (made outside any capture)
@@ -813,6 +815,13 @@ bool keeps_graph(const opfc_handle *h) { return h->plane || h->al_grad; }
 // Steps of one graph: a small grid's step is a few short kernels, so the gap
 // between graph launches would be a good part of it.
 constexpr int kGraphSteps = 10;
+
+// Large grids whose captured step does not outlive the field (from 2^21 cells on)
+// launch their first steps directly: a capture takes 0.13 ms and a graph saves 2 to
+// 15 us a step there (256^3 FP32 172 / 170, 512^3 1151 / 1134, 64x1024x256 196 /
+// 186), so it has paid for itself after about this many.
+constexpr size_t kEagerCells = (size_t)1 << 21;
+constexpr int kEagerSteps = 32;
 
 int build_graph(opfc_handle *h, int steps, cudaGraphExec_t *exec) {
   CUDA_TRY(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
@@ -1694,10 +1703,13 @@ int opfc_step(opfc_handle *h, int n_steps) {
     }
     return OPFC_OK;
   }
-  // From 2^21 cells on the separate passes are long enough to hide their launches.
-  const bool eager = !keeps_graph(h) && h->nr >= ((size_t)1 << 21);
+  const bool eager = !keeps_graph(h) && h->nr >= kEagerCells && !h->graph_exec &&
+                     n_steps <= kEagerSteps - h->eager_steps;
   if ((eager ? n_steps > 1 : keeps_graph(h) && n_steps >= kGraphSteps) && (rc = ensure_side(h))) return rc;
-  if (eager) return enqueue_steps(h, n_steps);
+  if (eager) {
+    h->eager_steps += n_steps;
+    return enqueue_steps(h, n_steps);
+  }
   while (n_steps > 0) {
     const bool many = keeps_graph(h) && n_steps >= kGraphSteps;
     cudaGraphExec_t *g = many ? &h->graph_many : &h->graph_exec;

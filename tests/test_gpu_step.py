@@ -168,3 +168,26 @@ def test_nvtx_eager_steps_match_oracle(oracle, monkeypatch):
     ref = oracle.run_plain(psi0, PI4, -0.25, 0.5, 6)
     _, psi = run_plain(n, ob.FP64, psi0, 6)
     assert rel_l2(psi, ref) <= 1e-11
+
+
+def test_long_runs_from_direct_launches_to_a_graph(oracle, monkeypatch):
+    """From 2^21 cells on the first steps after a field is set are launched directly
+    and a long run goes on with a captured step: the same steps in any division, also
+    after another field (whose mean the captured step holds)."""
+    monkeypatch.setenv("OPENPFC_GPU_AUTOTUNE_MODE", "fallback_only")
+    monkeypatch.setenv("OPFC_PLANE", "0")
+    n = (128, 128, 128)
+    m = ob.PfcB200(n, [math.pi / 4] * 3, precision=ob.FP32)
+    m.initialize(0.5)
+    for n0 in (-0.285, -0.2):
+        psi0 = oracle.ic_noise(n, n0, 0.01, 5)
+        got = []
+        for parts in ((40,), (20, 20), (1,) * 40, (32, 8), (31, 2, 7)):
+            m.set_psi(psi0)
+            for k in parts:
+                m.step(k)
+            m.sync()
+            got.append(m.get_psi())
+        assert all(np.array_equal(g, got[0]) for g in got[1:])
+        ref = oracle.run_plain(psi0, [math.pi / 4] * 3, -0.25, 0.5, 40)
+        assert np.linalg.norm((got[0] - ref).ravel()) <= 1e-5 * np.linalg.norm(ref.ravel())
