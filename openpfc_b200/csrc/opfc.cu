@@ -956,21 +956,26 @@ int default_x(const opfc_handle *h) {
 
 // Folded tables (each read once for two tiles) in place of the streamed ones.
 // - Direct loads up to 128 points and on mixed lengths (64x512x96 FP32 pipelined
-//   102, direct 79; 192x96x80 FP64 101 / 66; 256x256x128 FP32 108 / 99;
-//   512x256x128 FP64 366 / 330), and on small grids up to 512 points (64x64x512
-//   FP32 43 / 39); from 2^25 cells on the pipelined kernel (equal at 2^24:
-//   512x256x128 FP32 185 / 185).
+//   102, direct 79; 192x96x80 FP64 101 / 66; 256x256x128 FP32 98 / 90; 512x256x128
+//   FP64 366 / 330), and on small grids up to 512 points (64x64x512 FP32 37 / 31);
+//   from 2^25 cells on the pipelined kernel (equal at 2^24: 512x256x128 FP32 178 /
+//   180).  Two fields in FP32 get there sooner, their update being bound by memory
+//   and not by latency (Tungsten, pipelined / direct): at 128 points from 2^23 cells
+//   (256x256x128 152 / 160, 1024x128x128 323 / 356; 256x128x128 78 / 75), at 256 and
+//   512 past 2^21 (48x256x256 84 / 90, 48x96x512 65 / 72; 64x64x512 47 / 43).
 // - At 256 points with ping-pong buffers, longer without: 256^3 FP64 337 with,
-//   339 without, Tungsten 488 / 497; 512^3 FP32 1167 / 1142, filtered
-//   256x128x512 FP64 403 / 354.
+//   339 without, Tungsten 488 / 497; 256^3 FP32 172 / 172, 64x512x256 117 / 118
+//   (streamed tables 171 and 122); 512^3 FP32 1167 / 1142, filtered 256x128x512
+//   FP64 403 / 354.
 // - Rows of 128 bytes at 1024 points where the kz planes are a megabyte or more
 //   apart (1024^3 filtered: 5.4 ms the pass, 64-byte rows 7.7); at 256 KB they
 //   lose (filtered 256x256x1024: 719 / 704).
 int default_z(const opfc_handle *h) {
   if (!h->fold_ops || h->slab) return 0;
-  if (!pow2(h->n2) || (h->n2 <= 128 && h->nr < ((size_t)1 << 25)) ||
-      (h->n2 <= 512 && h->nr < ((size_t)1 << 22)))
-    return 7;
+  const bool two32 = two_field(h->desc.model) && h->prec == OPFC_FP32;
+  const size_t direct128 = (size_t)1 << (two32 && h->n2 == 128 ? 23 : 25);
+  const size_t direct512 = two32 ? ((size_t)1 << 21) + 1 : (size_t)1 << 22;
+  if (!pow2(h->n2) || (h->n2 <= 128 && h->nr < direct128) || (h->n2 <= 512 && h->nr < direct512)) return 7;
   if (h->n2 <= 256) return 6;
   const bool one_field = h->desc.model == OPFC_MODEL_PLAIN || h->desc.model == OPFC_MODEL_FILTERED;
   return h->n2 == 1024 && one_field && (size_t)h->M * h->n1 * 2 * h->rsz >= ((size_t)1 << 20) ? 9 : 8;
