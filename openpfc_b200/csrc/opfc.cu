@@ -614,6 +614,8 @@ XLaunch x_fused(opfc_handle *h) {
   return X;
 }
 
+bool pow2(int n) { return (n & (n - 1)) == 0; }
+
 // Whether y inverse, x and y forward can run as one plane kernel, and whether
 // they do when neither the autotuner nor the environment chose.
 bool plane_ok(const opfc_handle *h) {
@@ -623,17 +625,34 @@ bool plane_ok(const opfc_handle *h) {
 // kernel wins up to about 150 modes (of all fields together) per plane and kz
 // plane.  On large grids the separate passes come close to the memory's rate,
 // and one or two latency-bound CTAs per SM do not: it stops at 2^22 cells of all
-// fields.  Measured per step, separate passes / plane kernel (us): 64x64x24
-// FP32 20.8 / 15.2, 128x128x128 42.5 / 39.1, 192x96x80 47 / 35, 128x256x128
-// 59 / 50, 256x48x256 FP64 73 / 68, but 128x128x32 FP32 20.8 / 23.3,
-// 256x128x16 21 / 39, 1024x48x64 54 / 66, 256x128x256 98 / 106, 96x96x1024 FP64
-// 240 / 255; Tungsten 160x80x96 FP64 78 / 58, 96x80x48 32.5 / 36.6, 128x96x256
-// FP32 63 / 71.
+// fields.  Measured per step, separate passes / plane kernel (us): 64x64x24 FP32
+// 22.6 / 15.4, 128x256x128 58.5 / 49.7, 64x512x128 77 / 54, 256x48x256 FP64 72 / 68,
+// but 256x128x16 FP32 22 / 39, 256x128x64 35 / 43, 1024x48x64 41 / 66, 256x128x256
+// 90 / 105, 96x96x512 FP64 117 / 124; Tungsten 160x80x96 FP64 60 / 58, 96x80x48 31 / 37,
+// 128x96x256 FP32 62 / 70.  The line is a rough one near its ends, against the
+// separate passes with their present defaults: it leaves out 64x512x96 FP32 (78 /
+// 57) and takes 64x256x64 FP32 (29 / 34) and 256x64x64 FP64 (29 / 33).
 bool plane_pays(const opfc_handle *h, int fields) {
   return fields * (h->M + 1) * h->n1 <= 150 * h->n2 && fields * h->nr <= ((size_t)1 << 22);
 }
+
+// FP32 steps inside that line where the plane kernel still loses, to the separate
+// passes and to what they took with streamed tables:
+// - two fields on rows of 24 and 40 values (20 and 24 values a thread, one or two
+//   threads a row): Tungsten 80x24x32 24.1 / 25.9, 48x40x32 22.6 / 26.7, 48x96x128
+//   30.8 / 34.5;
+// - mixed lengths, one CTA per SM, whose planes of some size take several turns of
+//   the chip: 80x64x512 45 / 58, 192x32x512 47 / 69, Tungsten 192x32x256 39 / 55;
+//   with 256 and 512 rows a plane the separate y passes lose more (48x256x256 68 / 60).
+bool plane_late(const opfc_handle *h, int fields) {
+  if (h->prec != OPFC_FP32 || fields > 2) return false;
+  const bool mixed = !pow2(h->M) || !pow2(h->n1);
+  return (fields == 2 && (h->M == 24 || h->M == 40)) ||
+         (mixed && h->n2 >= 256 && h->n1 <= 128 && fields * (h->M + 1) * h->n1 >= 2600);
+}
 bool plane_default(const opfc_handle *h) {
-  return h->use_tma && plane_ok(h) && plane_pays(h, plane_fields(x_fused(const_cast<opfc_handle *>(h)).model));
+  const int fields = plane_fields(x_fused(const_cast<opfc_handle *>(h)).model);
+  return h->use_tma && plane_ok(h) && plane_pays(h, fields) && !plane_late(h, fields);
 }
 
 // The transform's plane kernel: where it fits and no pass is forced.
@@ -935,8 +954,7 @@ bool direct_ok(const opfc_handle *h, const void *p, int dtype, int where) {
 
 // Variants of the passes when neither the autotuner nor the environment chose
 // (us a step, the other passes alike).
-bool pow2(int n) { return (n & (n - 1)) == 0; }
-
+//
 // Direct loads on short lines: the pipelined kernel keeps one CTA per SM, with
 // 20 or 24 values a thread on mixed lengths.  512x96x256 FP64 pipelined 351,
 // direct 265; 256^3 FP64 339 / 325; 256x256x128 FP32 108 / 103; but 256x256x512
@@ -949,7 +967,9 @@ int default_y(const opfc_handle *h) {
 }
 
 // Rows loaded straight into registers from 2^26 cells on at M = 256, FP32 (512^3:
-// 1142 staged, 1130); below that the staged rows win (256x256x512 311 / 326).
+// 1142 staged, 1130).  At M = 128 the staged rows win (256^3 172 / 178, 256x256x512
+// 311 / 326); at M = 256 on smaller grids the two are within 2% (512x512x128 347 /
+// 347, 512x128x256 158 / 156).
 int default_x(const opfc_handle *h) {
   return h->M == 256 && h->prec == OPFC_FP32 && h->nr >= ((size_t)1 << 26) ? 3 : 0;
 }
@@ -962,7 +982,8 @@ int default_x(const opfc_handle *h) {
 //   180).  Two fields in FP32 get there sooner, their update being bound by memory
 //   and not by latency (Tungsten, pipelined / direct): at 128 points from 2^23 cells
 //   (256x256x128 152 / 160, 1024x128x128 323 / 356; 256x128x128 78 / 75), at 256 and
-//   512 past 2^21 (48x256x256 84 / 90, 48x96x512 65 / 72; 64x64x512 47 / 43).
+//   512 past 2^21 (80x128x256 62 / 65; 64x64x512 47 / 43), on rows of 24 past 2^20
+//   (48x96x256 43 / 45, 48x96x512 65 / 72).
 // - At 256 points with ping-pong buffers, longer without: 256^3 FP64 337 with,
 //   339 without, Tungsten 488 / 497; 256^3 FP32 172 / 172, 64x512x256 117 / 118
 //   (streamed tables 171 and 122); 512^3 FP32 1167 / 1142, filtered 256x128x512
@@ -974,7 +995,8 @@ int default_z(const opfc_handle *h) {
   if (!h->fold_ops || h->slab) return 0;
   const bool two32 = two_field(h->desc.model) && h->prec == OPFC_FP32;
   const size_t direct128 = (size_t)1 << (two32 && h->n2 == 128 ? 23 : 25);
-  const size_t direct512 = two32 ? ((size_t)1 << 21) + 1 : (size_t)1 << 22;
+  // (rows of 24 leave a quarter of the direct kernel's 16-column tiles empty)
+  const size_t direct512 = !two32 ? (size_t)1 << 22 : h->M == 24 ? (size_t)1 << 20 : ((size_t)1 << 21) + 1;
   if (!pow2(h->n2) || (h->n2 <= 128 && h->nr < direct128) || (h->n2 <= 512 && h->nr < direct512)) return 7;
   if (h->n2 <= 256) return 6;
   const bool one_field = h->desc.model == OPFC_MODEL_PLAIN || h->desc.model == OPFC_MODEL_FILTERED;
