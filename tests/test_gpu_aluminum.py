@@ -88,6 +88,40 @@ def test_aluminum_moving_gradient_vs_oracle(oracle, prec, tol):
     assert np.abs(ref - base).max() > 1e-6
 
 
+# (n0, n1, n2): three and one row tiles in the x pass's shared memory (n0 = 1024: one),
+# mixed lengths, a row count that is no multiple of the tile's 16 or 8 rows
+GRADIENT_SHAPES = [(32, 32, 32), (48, 40, 16), (96, 24, 1), (512, 16, 4), (1024, 16, 2)]
+
+
+@pytest.mark.parametrize("plane", ["0", "1"])
+@pytest.mark.parametrize("prec,tol", [(ob.FP64, 1e-11), (ob.FP32, 1e-5)])
+@pytest.mark.parametrize("n", GRADIENT_SHAPES)
+def test_moving_gradient_in_the_x_pass_and_the_plane_kernel(oracle, monkeypatch, n, prec, tol, plane):
+    """Both ways of the three-field step (OPFC_PLANE=0: the fused x pass of its own;
+    1: the plane kernel where it fits), over the ten-step graph and single steps, then
+    a second field of another mean on the same handle, whose graphs are kept."""
+    monkeypatch.setenv("OPENPFC_GPU_AUTOTUNE_MODE", "fallback_only")
+    monkeypatch.setenv("OPFC_PLANE", plane)
+    vals = dict(G_grid=2.0, V_grid=0.5, q4_bar=0.787482, tau_const=0.3, m_xpos=5.0, x_initial=4.0, stabP=0.05)
+    p, op = params(), oracle.AluminumParams.test_case()
+    for k, v in vals.items():
+        setattr(p, k, v)
+        setattr(op, k, v)
+    origin = [-3.0, 0.0, 0.0]
+    m = ob.AluminumB200(n, [1.0] * 3, p, precision=prec, origin=origin)
+    m.initialize(1e-2)
+    if plane == "0":
+        assert m.kernels_per_step() == 6
+    for mean, t0 in ((-0.006, 0.3), (0.1, 1.7)):
+        psi0 = ob.ic_noise(n, mean, 0.05, 8)
+        m.set_psi(psi0)
+        m.set_time(t0, 1e-2)
+        m.step(12)
+        m.sync()
+        ref = oracle.run_aluminum(psi0, [1.0] * 3, origin, op, 1e-2, 12, t0=t0, dt_t=1e-2)
+        assert np.linalg.norm((m.get_psi() - ref).ravel()) <= tol * np.linalg.norm(ref.ravel())
+
+
 def test_plane_choice_is_cached_by_fields(tmp_path, monkeypatch):
     """A moving gradient adds a third field to the step: its choice between the
     passes and the plane kernel is kept apart from the two-field step's."""

@@ -1,5 +1,5 @@
-"""Uneven-size ensemble (one persistent kernel per stage, n-step CUDA graph)
-against the FP64 oracle, member by member.  Sides are drawn from
+"""Uneven-size ensemble (one persistent kernel per stage or the plane kernel and
+the z update, n-step CUDA graph) against the FP64 oracle, member by member.  Sides are drawn from
 {32, 48, 64, 80, 96}; r ~ U(-0.35, -0.10), n0 ~ U(-0.35, -0.20), noise
 U(-0.01, 0.01) -- the parameter-sweep configuration at a reduced member count."""
 import math
@@ -33,9 +33,12 @@ def rel_l2(a, b):
     return float(np.linalg.norm((a - b).ravel()) / np.linalg.norm(b.ravel()))
 
 
+@pytest.mark.parametrize("plane", ["0", "1"])
 @pytest.mark.parametrize("prec,tol", [(ob.FP64, 1e-11), (ob.FP32, 1e-5)])
 @pytest.mark.parametrize("cubes", [True, False])
-def test_ensemble_vs_oracle(oracle, prec, tol, cubes):
+def test_ensemble_vs_oracle(oracle, monkeypatch, prec, tol, cubes, plane):
+    """The separate stages (OPFC_PLANE=0) and the plane kernel (1)."""
+    monkeypatch.setenv("OPFC_PLANE", plane)
     ms = members(12, 7 if cubes else 8, cubes)
     e = ob.Ensemble(ms, precision=prec)
     e.initialize(0.5)

@@ -1,8 +1,7 @@
-"""Both kernel families against the oracle: the persistent TMA/bulk-copy-fed
-passes (default) and the direct-load passes (OPFC_NO_TMA=1, read at handle
-creation), for every model and both precisions."""
+"""Every kernel that a step may take against the oracle: the defaults, and each
+variant of the separate passes (persistent TMA/bulk-copy-fed and direct loads)
+forced, for the plain, filtered and Tungsten models in both precisions."""
 import math
-import os
 
 import numpy as np
 import pytest
@@ -14,65 +13,45 @@ pytestmark = pytest.mark.gpu
 PI4 = [math.pi / 4] * 3
 
 
-@pytest.fixture(params=["tma", "tma_radial", "direct", "computed", "direct_computed", "pingpong", "e32",
-                        "folded", "folded_direct", "folded_nopp", "folded_wide"])
+# the y, x and z variants of each path (OPFC_Y_VARIANT, ...), all as separate passes
+PATHS = {"tma": (0, 0, 0), "tma_radial": (0, 0, 1), "direct": (0, 0, 0), "direct_xyz": (1, 1, 2),
+         "computed": (2, 2, 3), "direct_computed": (0, 0, 4), "pingpong": (3, 3, 5), "e32": (4, 0, 0),
+         "folded": (3, 3, 6), "folded_direct": (0, 0, 7), "folded_nopp": (0, 4, 8), "folded_wide": (0, 0, 9)}
+
+
+@pytest.fixture(params=["default"] + list(PATHS))
 def path(request, monkeypatch):
-    """tma: pipelined kernels streaming the per-mode tables (default);
-    tma_radial: the z update reading radial operator tables (OPFC_Z_VARIANT=1,
-    isotropic grids; others fall back to tables);
+    """default: what a handle takes by itself (the plane kernel on small grids);
+    tma: pipelined kernels streaming the per-mode tables;
+    tma_radial: the z update reading radial operator tables (isotropic grids;
+    others fall back to tables);
     direct: direct-load kernels (OPFC_NO_TMA=1);
-    computed: pipelined z update computing its operators from k^2
-    (OPFC_Z_VARIANT=3), half-width y tiles (OPFC_Y_VARIANT=2) and the x pass
-    without the warp-square kernel (OPFC_X_VARIANT=2);
-    direct_computed: direct z update computing its operators (OPFC_Z_VARIANT=4);
-    pingpong: ping-pong FFT exchange buffers in the y pass and the computed
-    z update (OPFC_Y_VARIANT=3, OPFC_Z_VARIANT=5), and the x pass's warp-square
-    kernel with rows loaded straight into registers (OPFC_X_VARIANT=3);
-    e32: direct-load y pass with 32 values per thread (OPFC_Y_VARIANT=4;
-    other lengths keep their plan);
+    direct_xyz: the direct-load variants of the three passes;
+    computed: pipelined z update computing its operators from k^2, half-width y
+    tiles and the x pass without the warp-square kernel;
+    direct_computed: direct z update computing its operators;
+    pingpong: ping-pong FFT exchange buffers in the y pass and the computed z
+    update, and the x pass's warp-square kernel with rows loaded straight into
+    registers;
+    e32: direct-load y pass with 32 values per thread (other lengths keep their plan);
     folded: the z update reading the folded FP64-built tables with ping-pong
-    exchange buffers, with the ping-pong y pass and the register-loaded x pass
-    (OPFC_Y_VARIANT=3, OPFC_X_VARIANT=3, OPFC_Z_VARIANT=6);
-    folded_direct: direct-load z update on the folded tables (OPFC_Z_VARIANT=7);
-    folded_nopp: pipelined z update on the folded tables without ping-pong
-    buffers (OPFC_Z_VARIANT=8) with the register-loaded x pass prefetching the
-    next row (OPFC_X_VARIANT=4);
+    exchange buffers, with the ping-pong y pass and the register-loaded x pass;
+    folded_direct: direct-load z update on the folded tables;
+    folded_nopp: pipelined z update on the folded tables without ping-pong buffers
+    with the register-loaded x pass prefetching the next row;
     folded_wide: the z update on the folded tables with 128-byte tile rows
-    streamed through a two-slot box ring (OPFC_Z_VARIANT=9; z lengths other
-    than 1024 and the Tungsten model take the direct-load kernel).
+    streamed through a two-slot box ring (z lengths other than 1024 and the
+    Tungsten model take the direct-load kernel).
     The Tungsten model has no computed operators and falls back to tables."""
-    monkeypatch.delenv("OPFC_NO_TMA", raising=False)
-    monkeypatch.delenv("OPFC_Z_VARIANT", raising=False)
-    monkeypatch.delenv("OPFC_Y_VARIANT", raising=False)
-    monkeypatch.delenv("OPFC_X_VARIANT", raising=False)
+    for k in ("OPFC_NO_TMA", "OPFC_PLANE", "OPFC_Y_VARIANT", "OPFC_X_VARIANT", "OPFC_Z_VARIANT"):
+        monkeypatch.delenv(k, raising=False)
     monkeypatch.setenv("OPENPFC_GPU_AUTOTUNE_MODE", "fallback_only")
     if request.param == "direct":
         monkeypatch.setenv("OPFC_NO_TMA", "1")
-    elif request.param == "tma_radial":
-        monkeypatch.setenv("OPFC_Z_VARIANT", "1")
-    elif request.param == "computed":
-        monkeypatch.setenv("OPFC_Z_VARIANT", "3")
-        monkeypatch.setenv("OPFC_Y_VARIANT", "2")
-        monkeypatch.setenv("OPFC_X_VARIANT", "2")
-    elif request.param == "direct_computed":
-        monkeypatch.setenv("OPFC_Z_VARIANT", "4")
-    elif request.param == "pingpong":
-        monkeypatch.setenv("OPFC_Y_VARIANT", "3")
-        monkeypatch.setenv("OPFC_Z_VARIANT", "5")
-        monkeypatch.setenv("OPFC_X_VARIANT", "3")
-    elif request.param == "e32":
-        monkeypatch.setenv("OPFC_Y_VARIANT", "4")
-    elif request.param == "folded":
-        monkeypatch.setenv("OPFC_Y_VARIANT", "3")
-        monkeypatch.setenv("OPFC_X_VARIANT", "3")
-        monkeypatch.setenv("OPFC_Z_VARIANT", "6")
-    elif request.param == "folded_direct":
-        monkeypatch.setenv("OPFC_Z_VARIANT", "7")
-    elif request.param == "folded_nopp":
-        monkeypatch.setenv("OPFC_Z_VARIANT", "8")
-        monkeypatch.setenv("OPFC_X_VARIANT", "4")
-    elif request.param == "folded_wide":
-        monkeypatch.setenv("OPFC_Z_VARIANT", "9")
+    if request.param != "default":
+        monkeypatch.setenv("OPFC_PLANE", "0")
+        for k, v in zip(("OPFC_Y_VARIANT", "OPFC_X_VARIANT", "OPFC_Z_VARIANT"), PATHS[request.param]):
+            monkeypatch.setenv(k, str(v))
     return request.param
 
 

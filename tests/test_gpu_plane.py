@@ -1,7 +1,8 @@
 """The plane kernel (y inverse, x and y forward of one kz plane in shared memory)
-against the oracle: every model, both precisions, plane sides of every plan
-(powers of two and mixed lengths, one line per turn up to several), and the
-transform's own plane and z kernels.  Tolerances as in the other parity tests:
+against the oracle: the plain, filtered and Tungsten models (the Aluminum step is
+in test_gpu_aluminum.py), both precisions, plane sides of every plan (powers of
+two and mixed lengths, one line per turn up to several), the transform's own plane
+and z kernels, and the reverse step.  Tolerances as in the other parity tests:
 FP64 rounding over the steps, FP32 its own rounding level."""
 import math
 
@@ -97,10 +98,16 @@ def test_transform_device_buffers(oracle, n2, prec):
 
 
 @pytest.mark.parametrize("prec,tol", [(ob.FP64, 1e-10), (ob.FP32, 1e-4)])
-@pytest.mark.parametrize("n", [(32, 16, 32), (48, 40, 48), (64, 48, 80)])
-def test_adjoint_against_general_path(monkeypatch, n, prec, tol):
+@pytest.mark.parametrize("n,z", [((32, 16, 32), None), ((48, 40, 48), None), ((64, 48, 80), None),
+                                 ((32, 16, 256), 0), ((32, 16, 256), 6), ((32, 16, 256), 8), ((32, 16, 1024), 8),
+                                 ((32, 16, 1024), 9)])
+def test_adjoint_against_general_path(monkeypatch, n, z, prec, tol):
     """Two kernels a reverse step against the general reverse step (OPFC_PLANE=0):
-    the same sums in another order, over 7 steps with segments of 3, 3 and 1."""
+    the same sums in another order, over 7 steps with segments of 3, 3 and 1.  The
+    recomputation's z update reads one array and writes another, in the direct-load
+    kernel (by default here) and in the pipelined ones (z forced)."""
+    if z is not None:
+        monkeypatch.setenv("OPFC_Z_VARIANT", str(z))
     psi0 = ob.ic_noise(n, -0.285, 0.05, 8)
     w = ob.ic_noise(n, 0.0, 1.0, 9)
     got = []
