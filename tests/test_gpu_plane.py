@@ -180,11 +180,35 @@ def test_ensemble(oracle, prec):
         assert _rel(e.get_psi(i), oracle.run_plain(p, PI4, ms[i]["r"], 0.5, 10)) <= TOL[prec]
 
 
+@pytest.fixture
+def used_memory():
+    """Small pieces of device memory that have held something before (bytes 0x40, as
+    a double 32.5) and are free again, among others that are not."""
+    import ctypes
+
+    import torch
+
+    torch.zeros(1, device="cuda")
+    drv = ctypes.CDLL("libcuda.so.1")
+    pieces = []
+    for size in (512, 1024, 9480, 9480, 9480, 16384) * 64:
+        p = ctypes.c_uint64()
+        assert drv.cuMemAlloc_v2(ctypes.byref(p), ctypes.c_size_t(size)) == 0
+        assert drv.cuMemsetD8_v2(p, ctypes.c_ubyte(0x40), ctypes.c_size_t(size)) == 0
+        pieces.append(p)
+    torch.cuda.synchronize()
+    for p in pieces[::2]:
+        assert drv.cuMemFree_v2(p) == 0
+    yield
+    for p in pieces[1::2]:
+        assert drv.cuMemFree_v2(p) == 0
+
+
 @pytest.mark.parametrize("plane", ["1", "0"])
 @pytest.mark.parametrize("prec", [ob.FP64, ob.FP32])
-def test_field_through_passes(oracle, monkeypatch, plane, prec):
+def test_field_through_passes(oracle, monkeypatch, used_memory, plane, prec):
     """A field that came through opfc_pass keeps its mean in psi_hat, so the steps
-    add none: also where the handle's memory held another handle's mean before."""
+    add none: also where the handle's memory held something before."""
     import torch
 
     from openpfc_b200.sharded import ARRAY_REAL, PASS_XY_FORWARD, PASS_Z_FORWARD, _CudaArray
@@ -192,10 +216,6 @@ def test_field_through_passes(oracle, monkeypatch, plane, prec):
     monkeypatch.setenv("OPFC_PLANE", plane)
     n = (32, 16, 48)
     psi0 = ob.ic_noise(n, -0.285, 0.01, 14)
-    before = ob.PfcB200(n, PI4, r=-0.25, precision=prec)
-    before.initialize(0.5)
-    before.set_psi(ob.ic_noise(n, 0.7, 0.01, 15))
-    before.close()
     m = ob.PfcB200(n, PI4, r=-0.25, precision=prec)
     m.initialize(0.5)
     ptr = ob.lib().opfc_array(m.handle, ARRAY_REAL)
