@@ -636,15 +636,18 @@ bool plane_pays(const opfc_handle *h, int fields) {
   return fields * (h->M + 1) * h->n1 <= 150 * h->n2 && fields * h->nr <= ((size_t)1 << 22);
 }
 
-// FP32 steps inside that line where the plane kernel still loses, to the separate
-// passes and to what they took with streamed tables:
+// Steps inside that line where the plane kernel still loses, to the separate passes
+// and to what they took with streamed tables.  FP32:
 // - two fields on rows of 24 and 40 values (20 and 24 values a thread, one or two
 //   threads a row): Tungsten 80x24x32 24.1 / 25.9, 48x40x32 22.6 / 26.7, 48x96x128
 //   30.8 / 34.5;
 // - mixed lengths, one CTA per SM, whose planes of some size take several turns of
 //   the chip: 80x64x512 45 / 58, 192x32x512 47 / 69, Tungsten 192x32x256 39 / 55;
 //   with 256 and 512 rows a plane the separate y passes lose more (48x256x256 68 / 60).
+// In either precision: two fields on a plane that keeps a single warp busy (Tungsten
+// 48x24x16 FP64, single steps 26.7 / 30.8).
 bool plane_late(const opfc_handle *h, int fields) {
+  if (fields == 2 && plane_threads(h->M, h->n1, (int)h->rsz) <= 32) return true;
   if (h->prec != OPFC_FP32 || fields > 2) return false;
   const bool mixed = !pow2(h->M) || !pow2(h->n1);
   return (fields == 2 && (h->M == 24 || h->M == 40)) ||
@@ -2291,8 +2294,7 @@ const char *opfc_step_kernel_region(int k) { return (k >= 0 && k < kStepKernels)
 //            = sum_n (1/N) sum_k w_kx Re(conj(lambda_hat) (...)),
 // dopL/dr = -k^2 dt opL,  dopN/dr = dt^2 k^4 phi'(L dt),
 // accumulated in FP64 per reduction block on the device across all steps.
-// psi_n comes from re-running the forward step (the same CUDA graph) from the
-// nearest snapshot.
+// psi_n comes from re-running the forward step from the nearest snapshot.
 // ---------------------------------------------------------------------------
 
 // Nonlinearity of the step's model from u = psi and v = C psi (in real space,
@@ -2341,9 +2343,6 @@ __global__ void adj_add_kernel(Real *lam, const Real *x, size_t n) {
     lam[i] += x[i];
 }
 
-// U = opL lam_hat (in place over lam_hat), V = opN lam_hat (over n_hat, after
-// it is read), and (tar != nullptr) FP64 sums of w_kx Re(conj(lam_hat)(dA psi_hat
-// + dB n_hat)) added to this block's running partial.
 // r-derivatives of the tables, built where they are used (one FP64 exp and expm1
 // per mode; the host took milliseconds at 128^3 and copied them over):
 // d opL/dr = -k^2 dt e^{L dt}, d opN/dr = dt^2 k^4 phi'(L dt), phi(x) = (e^x - 1)/x
@@ -2366,6 +2365,9 @@ __global__ void adj_tables_kernel(Real *ar, Real *br, int M, int n1, int n2, lon
   }
 }
 
+// U = opL lam_hat (in place over lam_hat), V = opN lam_hat (over n_hat, after
+// it is read), and (tar != nullptr) FP64 sums of w_kx Re(conj(lam_hat)(dA psi_hat
+// + dB n_hat)) added to this block's running partial.
 template <typename Real>
 __global__ void adj_modes_kernel(typename opfc::Cx<Real>::T *lam_hat, const typename opfc::Cx<Real>::T *psi_hat,
                                  typename opfc::Cx<Real>::T *n_hat, const Real *ta, const Real *tb,
