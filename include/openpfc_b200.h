@@ -131,8 +131,9 @@ int opfc_get_psi_hat(opfc_handle *h, void *psi_hat, size_t count, int dtype, int
 int opfc_get_psi_mf(opfc_handle *h, void *psi_mf, size_t count, int dtype, int where);
 
 /* Advance n_steps time steps (Model::step, cpu/tungsten_model.hpp:306;
- * 10_complete_pfc_model.cpp:121).  Asynchronous on the handle's stream; the
- * step sequence is captured in a CUDA graph on first use. */
+ * 10_complete_pfc_model.cpp:121).  Asynchronous on the handle's stream.  Steps
+ * come from a captured CUDA graph; on large grids the first ones after a field is
+ * set are launched directly. */
 int opfc_step(opfc_handle *h, int n_steps);
 /* Wait for the handle's stream; reports OPFC_ERR_NONFINITE if any step
  * produced NaN/Inf since the last check. */
@@ -280,12 +281,13 @@ int opfc_variants(const opfc_handle *h, int *var);
 /* Uneven-size ensembles (no counterpart in the reference, which runs one field
  * per MPI job): `count` independent plain-PFC fields, each with its own size
  * (N0/2 in {16,24,32,40,48,64}, N1, N2 in {16,32,48,64,80,96,128}), dx and r,
- * one precision.  Every stage of a step is one persistent kernel over all
- * members; opfc_ensemble_step(n) captures the n-step loop as one CUDA graph.
+ * one precision.  Every stage of a step is one kernel over all members (the y, x
+ * and y passes one together where that is faster); opfc_ensemble_step(n) captures the n-step loop as one CUDA graph.
  * Fields are host FP64 arrays (x fastest).  opfc_ensemble_autotune times the
  * variants (tile width 16 / 8 lines x 4 / 8 / 16 CTAs per SM, which also sets
- * the kernel's register budget) of the y, x and z-update stages separately,
- * reports 6 milliseconds per stage, caches the fastest (see
+ * the kernel's register budget) of the y, x and z-update stages separately, and
+ * the y, x and y stages against the plane kernel,
+ * reports 6 milliseconds per y, x and z stage, caches the fastest (see
  * OPENPFC_GPU_AUTOTUNE_* in the library notes) and invalidates the states. */
 typedef struct opfc_ensemble opfc_ensemble;
 int opfc_ensemble_create(int count, const opfc_desc *descs, opfc_ensemble **out);

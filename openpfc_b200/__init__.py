@@ -458,7 +458,7 @@ def ic_seeds(n, dx, n0, noise, nseeds, radius_cells, amp, seed) -> np.ndarray:
 
 class Ensemble:
     """Independent plain-PFC fields of different sizes and parameters advanced
-    together: one persistent kernel per stage, the step loop in one CUDA graph.
+    together: one kernel per stage over all of them, the step loop in one CUDA graph.
 
     members: sequence of dicts with keys n (N0, N1, N2), dx (3 values), r."""
 

@@ -1,6 +1,7 @@
 // ens_plane.cuh -- y inverse, fused x pass and y forward of an ensemble, one
 // member's kz plane per CTA (plane.cuh): one launch and one read and write of the
-// spectra in place of three.
+// spectra in place of three.  Used where that was measured to win (plane_pays in
+// ensemble.cu: 64 cubes of 64 FP32 248 to 214 us a step).
 //
 // Members' planes are at most 65 x 128 modes, so every one fits.  Blocks have
 // 288 threads: 36 lines of a 64-point column (33 are needed), 72 of an 80- or

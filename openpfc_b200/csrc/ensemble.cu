@@ -560,7 +560,7 @@ int opfc_ensemble_step(opfc_ensemble *e, int n_steps) {
   if (n_steps == 0) return OPFC_OK;  // step(0) only prepares the work arrays
   if (!e->graph || e->graph_steps != n_steps) {
     drop_graph(e);
-    // the whole n-step loop is one graph: 5 kernels per step
+    // the whole n-step loop is one graph: 5 kernels per step, 3 with the plane kernel
     ECUDA(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
     rc = enqueue_steps(e, n_steps);
     cudaGraph_t g = nullptr;
