@@ -18,15 +18,27 @@ import torch
 from . import FP64, PfcB200
 
 
+def _order(model, t: torch.Tensor, before: bool):
+    """The model works on a stream of its own: what torch has queued for `t` comes
+    before the model's next work, or the model's last work before torch's next."""
+    if t.is_cuda:
+        own, here = torch.cuda.ExternalStream(model.stream, device=t.device), torch.cuda.current_stream(t.device)
+        (own if before else here).wait_stream(here if before else own)
+
+
 class PfcEvolve(torch.autograd.Function):
     @staticmethod
     def forward(ctx, psi0: torch.Tensor, r, model, n_steps: int, K: int = 20):
         if r is not None:
             model.set_r(float(r))
-        model.set_psi(psi0.detach().contiguous())
+        psi0 = psi0.detach().contiguous()
+        _order(model, psi0, before=True)
+        model.set_psi(psi0)
         model.forward_checkpointed(n_steps, K)
         out = torch.empty_like(psi0)
+        _order(model, out, before=True)  # out's memory may still be in use
         model.get_psi(out)
+        _order(model, out, before=False)
         ctx.model = model
         ctx.has_r = r is not None
         ctx.r_dtype = r.dtype if r is not None else None
@@ -35,7 +47,10 @@ class PfcEvolve(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_out: torch.Tensor):
-        g0, gr, _ = ctx.model.adjoint(grad_out.detach().contiguous())
+        grad_out = grad_out.detach().contiguous()
+        g0 = torch.zeros_like(grad_out)
+        _order(ctx.model, grad_out, before=True)
+        g0, gr, _ = ctx.model.adjoint(grad_out, g0)
         g_r = torch.tensor(gr, dtype=ctx.r_dtype, device=ctx.r_device) if ctx.has_r else None
         return g0, g_r, None, None, None
 

@@ -91,6 +91,36 @@ def test_autograd_function_matches_adjoint():
     assert abs(float(r.grad) - gr) <= 1e-10 * abs(gr)
 
 
+def test_autograd_function_orders_its_stream_with_torch():
+    """psi0 and the gradient may still be being computed when they are passed, and the
+    results are used at once: the model's stream waits for torch's and torch's for it."""
+    import torch
+    from openpfc_b200.autograd import PfcEvolve, make_model
+    n = (128, 128, 64)
+    base = torch.tensor(ob.ic_noise(n, -0.285, 0.01, 5), device="cuda")
+    weight = torch.tensor(ob.ic_noise(n, 0.0, 1.0, 6), device="cuda")
+    model = make_model(n, PI4, precision=ob.FP64, dt=DT)
+    got = []
+    for late in (False, True):
+        torch.cuda.synchronize()
+        if late:
+            torch.cuda._sleep(20_000_000)  # some ms of a waiting kernel before each input
+        psi0 = (base * 1.0).requires_grad_()
+        psi = PfcEvolve.apply(psi0, None, model, 4, 2)
+        now = psi.detach().clone()
+        if late:
+            torch.cuda._sleep(20_000_000)
+        (g,) = torch.autograd.grad(psi, psi0, weight * 1.0)
+        g = g.clone()
+        torch.cuda.synchronize()
+        got.append((now.cpu(), g.cpu()))
+        del psi0, psi
+        base2 = torch.full_like(base, 7.0)  # what reused memory would hold
+        del base2
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
 def test_set_r_after_a_failed_rebuild(oracle):
     """A rebuild of the tables that fails (here: its synchronous copies are refused
     while a stream capture is open) leaves no tables to step with, and the same r
