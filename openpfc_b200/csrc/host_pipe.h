@@ -43,6 +43,7 @@ class HostPipe {
   static constexpr size_t kShareBytes = size_t(1) << 20;  // device bytes that are worth a thread
   static constexpr size_t kMinSlot = size_t(1) << 18, kMaxSlot = size_t(1) << 20;
   static constexpr size_t kOneCopy = size_t(1) << 26;
+  static constexpr size_t kPinAtOnce = size_t(1) << 24;
   static constexpr int kMaxThreads = 16;
 
   ~HostPipe() { release(); }
@@ -60,7 +61,7 @@ class HostPipe {
   cudaError_t in(int device, const H *src, D *dst, size_t n, cudaStream_t s, std::vector<double> *parts) {
     if (std::is_same<H, D>::value && !parts && one_copy(src, n * sizeof(D)))
       return cudaMemcpyAsync(dst, src, n * sizeof(D), cudaMemcpyHostToDevice, s);
-    return run<D>(device, n, s, parts, [=](size_t lo, size_t hi, D *const *slot, cudaEvent_t *ev, LaneSum *sum) {
+    return run<D>(device, n, s, false, parts, [=](size_t lo, size_t hi, D *const *slot, cudaEvent_t *ev, LaneSum *sum) {
       const size_t step = slot_ / sizeof(D);
       cudaError_t e = cudaSuccess;
       int k = 0;
@@ -84,7 +85,11 @@ class HostPipe {
       const cudaError_t e = cudaMemcpyAsync(dst, src, n * sizeof(D), cudaMemcpyDeviceToHost, s);
       return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
     }
-    return run<D>(device, n, s, nullptr, [=](size_t lo, size_t hi, D *const *slot, cudaEvent_t *ev, LaneSum *) {
+    // Copies into ordinary slots are slow (16 MiB through them 5.8 ms, through
+    // pinned ones 0.9): the second array out pins, the first goes as one copy into a
+    // temporary, as handles often read out once (2.6 ms; pinning alone takes 3 to 5).
+    if (std::max(n * sizeof(D), expect_) <= kPinAtOnce && !pinned_ && outs_++ == 0) return out_once(src, dst, n, s);
+    return run<D>(device, n, s, true, nullptr, [=](size_t lo, size_t hi, D *const *slot, cudaEvent_t *ev, LaneSum *) {
       const size_t step = slot_ / sizeof(D);
       cudaError_t e = cudaSuccess;
       auto issue = [&](size_t i, int k) {
@@ -127,6 +132,7 @@ class HostPipe {
   int threads_ = 0;  // threads with slots and events
   size_t slot_ = 0;  // bytes of a slot
   size_t expect_ = 0;
+  int outs_ = 0;  // arrays out while the slots were not pinned
   std::vector<cudaEvent_t> ev_;
 
   template <typename A, typename B> static void convert(const A *a, B *b, size_t n) {
@@ -148,16 +154,18 @@ class HostPipe {
     return (int)std::min<size_t>({(size_t)kMaxThreads, cores, std::max<size_t>(1, (bytes + kShareBytes - 1) / kShareBytes)});
   }
 
-  // Slots and events for arrays of `bytes`.  Pinning costs 0.6 ms a MiB, once: a
-  // slot holds a sixteenth of a thread's share (256 KiB to 1 MiB), and an array of
-  // one share goes through ordinary memory (256 KiB of FP32 from FP64: 0.08 ms
-  // either way, but 1.5 ms for the first call with pinned slots).
-  cudaError_t ensure(size_t bytes) {
+  // Slots and events for arrays of `bytes`, each slot a sixteenth of a thread's
+  // share (256 KiB to 1 MiB).  Pinning costs 3 ms and 0.3 to 0.6 ms a MiB, once for
+  // a handle: large arrays repay it in one call, others are copied in from ordinary
+  // memory at the same rate (128^3 FP32 from FP64: 1.0 to 2.3 ms either way) and
+  // pinned for the way out only, where it matters (`pin`).
+  cudaError_t ensure(size_t bytes, bool pin) {
     bytes = std::max(bytes, expect_);
+    pin = bytes > kPinAtOnce || (pin && bytes > kShareBytes);
     const int threads = threads_for(bytes);
-    const bool pin = bytes > kShareBytes;
-    const size_t slot = pin ? std::min(kMaxSlot, std::max(kMinSlot, (bytes / threads / 16 + 4095) / 4096 * 4096)) : kMaxSlot;
-    if (threads <= threads_ && (!pin || (tried_pin_ && slot <= slot_))) return cudaSuccess;
+    const size_t sixteenth = (bytes / threads / 16 + 4095) / 4096 * 4096;
+    const size_t slot = threads == 1 ? kMaxSlot : std::min(kMaxSlot, std::max(kMinSlot, sixteenth));
+    if (threads <= threads_ && slot <= slot_ && (!pin || tried_pin_)) return cudaSuccess;
     for (cudaEvent_t e : ev_) cudaEventSynchronize(e);  // copies out of the old slots
     release();
     cudaError_t e = cudaSuccess;
@@ -181,23 +189,10 @@ class HostPipe {
     return cudaSuccess;
   }
 
-  // f(lo, hi, slots, events, sum) on each thread's share of n values of D.  The
-  // per-thread default stream is another stream on every thread: the caller's own
-  // thread then does it all.
-  template <typename D, typename F>
-  cudaError_t run(int device, size_t n, cudaStream_t s, std::vector<double> *parts, const F &f) {
-    const int T = s == cudaStreamPerThread ? 1 : threads_for(n * sizeof(D));
-    cudaError_t e = ensure(n * sizeof(D));
-    if (e != cudaSuccess) return e;
-    const size_t share = ((n + T - 1) / T + 3) / 4 * 4;
-    std::vector<cudaError_t> rc(T, cudaSuccess);
-    std::vector<LaneSum> sums(parts ? T : 0);
-    auto work = [&](int t) {
-      const size_t lo = std::min(n, share * t), hi = std::min(n, lo + share);
-      D *slot[2] = {reinterpret_cast<D *>(pin_ + 2 * t * slot_), reinterpret_cast<D *>(pin_ + (2 * t + 1) * slot_)};
-      rc[t] = cudaSetDevice(device);
-      if (rc[t] == cudaSuccess) rc[t] = f(lo, hi, slot, &ev_[2 * t], parts ? &sums[t] : nullptr);
-    };
+  // f(t, lo, hi) on T threads, this one included, for their shares of n values
+  template <typename F> static void share(int T, size_t n, const F &f) {
+    const size_t each = ((n + T - 1) / T + 3) / 4 * 4;
+    auto work = [&](int t) { f(t, std::min(n, each * t), std::min(n, each * t + each)); };
     std::vector<std::thread> th;
     th.reserve(T);
     int started = 1;  // share 0 runs here
@@ -208,6 +203,34 @@ class HostPipe {
     work(0);
     for (int t = started; t < T; ++t) work(t);
     for (auto &x : th) x.join();
+  }
+
+  template <typename D, typename H> static cudaError_t out_once(const D *src, H *dst, size_t n, cudaStream_t s) {
+    D *tmp = static_cast<D *>(std::malloc(n * sizeof(D)));
+    if (!tmp) return cudaErrorMemoryAllocation;
+    cudaError_t e = cudaMemcpyAsync(tmp, src, n * sizeof(D), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess)
+      share(threads_for(n * sizeof(D)), n, [&](int, size_t lo, size_t hi) { convert(tmp + lo, dst + lo, hi - lo); });
+    std::free(tmp);
+    return e;
+  }
+
+  // f(lo, hi, slots, events, sum) on each thread's share of n values of D.  The
+  // per-thread default stream is another stream on every thread: the caller's own
+  // thread then does it all.
+  template <typename D, typename F>
+  cudaError_t run(int device, size_t n, cudaStream_t s, bool pin, std::vector<double> *parts, const F &f) {
+    const int T = s == cudaStreamPerThread ? 1 : threads_for(n * sizeof(D));
+    cudaError_t e = ensure(n * sizeof(D), pin);
+    if (e != cudaSuccess) return e;
+    std::vector<cudaError_t> rc(T, cudaSuccess);
+    std::vector<LaneSum> sums(parts ? T : 0);
+    share(T, n, [&](int t, size_t lo, size_t hi) {
+      D *slot[2] = {reinterpret_cast<D *>(pin_ + 2 * t * slot_), reinterpret_cast<D *>(pin_ + (2 * t + 1) * slot_)};
+      rc[t] = cudaSetDevice(device);
+      if (rc[t] == cudaSuccess) rc[t] = f(lo, hi, slot, &ev_[2 * t], parts ? &sums[t] : nullptr);
+    });
     for (cudaError_t r : rc)
       if (r != cudaSuccess) return r;
     if (parts)
