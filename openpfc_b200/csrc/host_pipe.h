@@ -1,9 +1,9 @@
 // host_pipe.h -- host arrays in and out of device buffers, with conversion.
 //
 // The arrays that a program passes are ordinary pageable memory, often in
-// another precision than the handle's.  A pipe owns pinned slots, two per host
-// thread; each thread converts its own share of the array slot by slot while
-// its previous slot is being copied, so conversion, page faults of a fresh
+// another precision than the handle's.  A pipe owns slots, two per host thread,
+// pinned where that pays; each thread converts its own share of the array slot by
+// slot while its previous slot is being copied, so conversion, page faults of a fresh
 // destination and the copy overlap and spread over the cores.  (Converting a
 // 256^3 FP64 array on one thread into a temporary and copying that pageable
 // temporary took most of 131 ms for set, 100 steps and get; with the pipe the
