@@ -18,12 +18,14 @@ import torch
 from . import FP64, PfcB200
 
 
-def _order(model, t: torch.Tensor, before: bool):
-    """The model works on a stream of its own: what torch has queued for `t` comes
-    before the model's next work, or the model's last work before torch's next."""
-    if t.is_cuda:
-        own, here = torch.cuda.ExternalStream(model.stream, device=t.device), torch.cuda.current_stream(t.device)
-        (own if before else here).wait_stream(here if before else own)
+def _streams(model, t: torch.Tensor):
+    """(the model's stream, torch's current one) for a device tensor, else None."""
+    if not t.is_cuda:
+        return None
+    own = getattr(model, "_torch_stream", None)
+    if own is None:
+        own = model._torch_stream = torch.cuda.ExternalStream(model.stream, device=t.device)
+    return own, torch.cuda.current_stream(t.device)
 
 
 class PfcEvolve(torch.autograd.Function):
@@ -32,13 +34,17 @@ class PfcEvolve(torch.autograd.Function):
         if r is not None:
             model.set_r(float(r))
         psi0 = psi0.detach().contiguous()
-        _order(model, psi0, before=True)
+        out = torch.empty_like(psi0)
+        # the model works on a stream of its own: after what torch has queued for psi0
+        # and on out's memory, and before what torch does with out
+        s = _streams(model, psi0)
+        if s:
+            s[0].wait_stream(s[1])
         model.set_psi(psi0)
         model.forward_checkpointed(n_steps, K)
-        out = torch.empty_like(psi0)
-        _order(model, out, before=True)  # out's memory may still be in use
         model.get_psi(out)
-        _order(model, out, before=False)
+        if s:
+            s[1].wait_stream(s[0])
         ctx.model = model
         ctx.has_r = r is not None
         ctx.r_dtype = r.dtype if r is not None else None
@@ -48,8 +54,10 @@ class PfcEvolve(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_out: torch.Tensor):
         grad_out = grad_out.detach().contiguous()
-        g0 = torch.zeros_like(grad_out)
-        _order(ctx.model, grad_out, before=True)
+        g0 = torch.empty_like(grad_out)
+        s = _streams(ctx.model, grad_out)
+        if s:
+            s[0].wait_stream(s[1])
         g0, gr, _ = ctx.model.adjoint(grad_out, g0)
         g_r = torch.tensor(gr, dtype=ctx.r_dtype, device=ctx.r_device) if ctx.has_r else None
         return g0, g_r, None, None, None

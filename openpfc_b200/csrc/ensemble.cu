@@ -461,7 +461,7 @@ int opfc_ensemble_create(int count, const opfc_desc *descs, opfc_ensemble **out)
       if (cudaEventCreateWithFlags(&v, cudaEventDisableTiming) != cudaSuccess) return bail(OPFC_ERR_CUDA);
     ep->plane = plane_choice(AutoTuner::instance().get_config(e->key + "/xy", plane_pays(ep)) == 1);
   }
-  ep->pipe.expect(ep->nr_max * ep->rsz);
+  ep->pipe.expect(ep->nr_max * ep->rsz, count);
   if (cudaMemset(ep->flag, 0, sizeof(unsigned)) != cudaSuccess || cudaMemset(ep->psi_hat, 0, cb) != cudaSuccess ||
       cudaMemset(ep->work, 0, cb) != cudaSuccess)
     return bail(OPFC_ERR_CUDA);

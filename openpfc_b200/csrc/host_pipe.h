@@ -14,10 +14,10 @@
 // and 14.2).
 #pragma once
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <algorithm>
 #include <cmath>
-#include <cstdlib>
 #include <cstring>
 #include <thread>
 #include <type_traits>
@@ -26,6 +26,16 @@
 #include "user_buffer.h"
 
 namespace opfc {
+
+// Pages of ordinary memory, from the system and back to it: a large block freed to
+// the C library would raise the size from which it maps blocks, for the program's
+// own arrays too.
+inline void *map_pages(size_t bytes) {
+  void *p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+  if (p == MAP_FAILED) return nullptr;
+  madvise(p, bytes, MADV_HUGEPAGE);  // fewer faults; where it is refused, ordinary pages
+  return p;
+}
 
 // running compensated (Neumaier) sum in four independent lanes, so that the
 // additions of one element do not wait for those of the one before
@@ -41,17 +51,22 @@ struct LaneSum {
 class HostPipe {
  public:
   static constexpr size_t kShareBytes = size_t(1) << 20;  // device bytes that are worth a thread
-  static constexpr size_t kMinSlot = size_t(1) << 18, kMaxSlot = size_t(1) << 20;
-  static constexpr size_t kOneCopy = size_t(1) << 26;
-  static constexpr size_t kPinAtOnce = size_t(1) << 24;
+  static constexpr size_t kMinSlot = size_t(1) << 19, kMaxSlot = size_t(1) << 20;
+  static constexpr size_t kNeverPin = size_t(1) << 17, kPinAtOnce = size_t(1) << 25;
+  static constexpr size_t kOneCopyFrom = size_t(4) << 20, kOneCopyTo = size_t(20) << 20;
   static constexpr int kMaxThreads = 16;
 
   ~HostPipe() { release(); }
 
-  // slots for arrays of up to `bytes` device bytes from the first one on: an
-  // ensemble's members come in any order, and slots pinned again as they grow are
-  // paid for each time (setting 64 members: 50 ms so, 36 with one set of slots)
-  void expect(size_t bytes) { expect_ = bytes; }
+  // an ensemble's `arrays` of up to `bytes` device bytes: they come in any order, and
+  // slots that grow with them are paid for each time (setting 64 members: 50 ms so, 36
+  // with one set of slots).  A few are all read out once before the slots are pinned
+  // (8 members 2.6 ms so, 21 with the pinning), many repay it in their first round (64
+  // members 50 ms, 70 to 86 without).
+  void expect(size_t bytes, int arrays) {
+    expect_ = bytes;
+    once_ = arrays < 16 ? arrays : 1;
+  }
 
   // n values host (H) -> device (D) on stream s; with `parts`, the compensated
   // sums of the host values are appended to it.  Returns before the last copies
@@ -59,7 +74,7 @@ class HostPipe {
   // that goes as one copy has to stay as it is until then).
   template <typename H, typename D>
   cudaError_t in(int device, const H *src, D *dst, size_t n, cudaStream_t s, std::vector<double> *parts) {
-    if (std::is_same<H, D>::value && !parts && one_copy(src, n * sizeof(D)))
+    if (std::is_same<H, D>::value && !parts && one_copy_in(src, n * sizeof(D)))
       return cudaMemcpyAsync(dst, src, n * sizeof(D), cudaMemcpyHostToDevice, s);
     return run<D>(device, n, s, false, parts, [=](size_t lo, size_t hi, D *const *slot, cudaEvent_t *ev, LaneSum *sum) {
       const size_t step = slot_ / sizeof(D);
@@ -81,14 +96,14 @@ class HostPipe {
   // n values device (D) -> host (H), complete on return
   template <typename D, typename H>
   cudaError_t out(int device, const D *src, H *dst, size_t n, cudaStream_t s) {
-    if (std::is_same<H, D>::value && one_copy(dst, n * sizeof(D))) {
+    const bool same = std::is_same<H, D>::value;
+    const size_t bytes = std::max(n * sizeof(D), expect_);
+    const bool first = !pinned_ && bytes <= kPinAtOnce && outs_++ < once_;
+    if (same && (first || pinned_host_memory(pointer_attributes(dst)))) {
       const cudaError_t e = cudaMemcpyAsync(dst, src, n * sizeof(D), cudaMemcpyDeviceToHost, s);
       return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
     }
-    // Copies into ordinary slots are slow (16 MiB through them 5.8 ms, through
-    // pinned ones 0.9): the second array out pins, the first goes as one copy into a
-    // temporary, as handles often read out once (2.6 ms; pinning alone takes 3 to 5).
-    if (std::max(n * sizeof(D), expect_) <= kPinAtOnce && !pinned_ && outs_++ == 0) return out_once(src, dst, n, s);
+    if (first) return out_once(src, dst, n, s);
     return run<D>(device, n, s, true, nullptr, [=](size_t lo, size_t hi, D *const *slot, cudaEvent_t *ev, LaneSum *) {
       const size_t step = slot_ / sizeof(D);
       cudaError_t e = cudaSuccess;
@@ -117,8 +132,8 @@ class HostPipe {
     ev_.clear();
     if (pin_ && pinned_)
       cudaFreeHost(pin_);
-    else
-      std::free(pin_);
+    else if (pin_)
+      munmap(pin_, pin_bytes_);
     pin_ = nullptr;
     pinned_ = tried_pin_ = false;
     threads_ = 0;
@@ -127,12 +142,13 @@ class HostPipe {
 
  private:
   char *pin_ = nullptr;
+  size_t pin_bytes_ = 0;
   bool tried_pin_ = false;  // the slots are pinned, or pinning was refused
   bool pinned_ = false;  // else pageable: the copies are then slower and synchronous, with the same result
   int threads_ = 0;  // threads with slots and events
   size_t slot_ = 0;  // bytes of a slot
   size_t expect_ = 0;
-  int outs_ = 0;  // arrays out while the slots were not pinned
+  int outs_ = 0, once_ = 1;  // arrays out while the slots were not pinned, and how many go so
   std::vector<cudaEvent_t> ev_;
 
   template <typename A, typename B> static void convert(const A *a, B *b, size_t n) {
@@ -142,11 +158,13 @@ class HostPipe {
       for (size_t i = 0; i < n; ++i) b[i] = (B)a[i];
   }
 
-  // An array without conversion that no staging would speed up: pinned, or no
-  // larger than kOneCopy (64 MiB: 5.4 to 6.3 ms in as one copy, 4.0 to 4.3 through
-  // slots that cost 5 ms to pin; 512 MiB: 50 and 15).
-  static bool one_copy(const void *host, size_t bytes) {
-    return bytes <= kOneCopy || pinned_host_memory(pointer_attributes(host));
+  // Whether an array without conversion goes in as one copy: pinned, or the slots
+  // are not pinned, or of a size that staging does not speed up (128x64x64 FP64 0.32 ms
+  // so, 0.43 through pinned slots; 128^3 1.1 and 1.4; but 256x256x128 5.4 and 4.0, and
+  // at 64^3 0.21 either way with the next array out 0.35 and 0.23, its threads being
+  // warm).
+  bool one_copy_in(const void *host, size_t bytes) const {
+    return !pinned_ || (bytes >= kOneCopyFrom && bytes < kOneCopyTo) || pinned_host_memory(pointer_attributes(host));
   }
 
   static int threads_for(size_t bytes) {
@@ -154,28 +172,34 @@ class HostPipe {
     return (int)std::min<size_t>({(size_t)kMaxThreads, cores, std::max<size_t>(1, (bytes + kShareBytes - 1) / kShareBytes)});
   }
 
-  // Slots and events for arrays of `bytes`, each slot a sixteenth of a thread's
-  // share (256 KiB to 1 MiB).  Pinning costs 3 ms and 0.3 to 0.6 ms a MiB, once for
-  // a handle: large arrays repay it in one call, others are copied in from ordinary
-  // memory at the same rate (128^3 FP32 from FP64: 1.0 to 2.3 ms either way) and
-  // pinned for the way out only, where it matters (`pin`).
+  // Slots and events for arrays of `bytes`: a slot holds an eighth of a thread's share
+  // (512 KiB to 1 MiB; through 256 KiB slots 64 MiB out took 3.3 ms, 2.0 so), or one
+  // thread's array.  Pinning costs 2 to 3 ms and 0.3 to
+  // 0.6 ms a MiB, once for a handle.  Arrays in go through ordinary slots at nearly
+  // the same rate (128^3 FP32 from FP64 1.0 to 2.3 ms either way).  Arrays out are
+  // much faster through pinned ones, most of all into fresh pages (FP64, one copy /
+  // pinned slots: 64x16x24 78 / 42 us, 64^3 360 / 223, 128^3 2200 / 1450, 256x256x128
+  // 14.8 / 2.7 ms), so the second array out pins (a small ensemble's second round): the
+  // first goes as one copy, into a temporary where it needs conversion, as handles are
+  // often read out once.  Arrays of more than 32 MiB repay the pinning at once.
   cudaError_t ensure(size_t bytes, bool pin) {
     bytes = std::max(bytes, expect_);
-    pin = bytes > kPinAtOnce || (pin && bytes > kShareBytes);
+    pin = pin && bytes > kNeverPin;
     const int threads = threads_for(bytes);
-    const size_t sixteenth = (bytes / threads / 16 + 4095) / 4096 * 4096;
-    const size_t slot = threads == 1 ? kMaxSlot : std::min(kMaxSlot, std::max(kMinSlot, sixteenth));
+    const size_t part = threads == 1 ? bytes : std::max(kMinSlot, bytes / threads / 8);
+    const size_t slot = std::min(kMaxSlot, (part + 4095) / 4096 * 4096);
     if (threads <= threads_ && slot <= slot_ && (!pin || tried_pin_)) return cudaSuccess;
     for (cudaEvent_t e : ev_) cudaEventSynchronize(e);  // copies out of the old slots
     release();
     cudaError_t e = cudaSuccess;
+    pin_bytes_ = 2 * slot * threads;
     if (pin) {
-      e = cudaHostAlloc((void **)&pin_, 2 * slot * threads, cudaHostAllocDefault);
+      e = cudaHostAlloc((void **)&pin_, pin_bytes_, cudaHostAllocDefault);
       if (e != cudaSuccess) cudaGetLastError();
       tried_pin_ = true;
     }
     pinned_ = pin && e == cudaSuccess;
-    if (!pinned_ && !(pin_ = static_cast<char *>(std::malloc(2 * slot * threads)))) return cudaErrorMemoryAllocation;
+    if (!pinned_ && !(pin_ = static_cast<char *>(map_pages(pin_bytes_)))) return cudaErrorMemoryAllocation;
     slot_ = slot;
     for (int i = 0; i < 2 * threads; ++i) {
       cudaEvent_t v = nullptr;
@@ -206,13 +230,13 @@ class HostPipe {
   }
 
   template <typename D, typename H> static cudaError_t out_once(const D *src, H *dst, size_t n, cudaStream_t s) {
-    D *tmp = static_cast<D *>(std::malloc(n * sizeof(D)));
+    D *tmp = static_cast<D *>(map_pages(n * sizeof(D)));
     if (!tmp) return cudaErrorMemoryAllocation;
     cudaError_t e = cudaMemcpyAsync(tmp, src, n * sizeof(D), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e == cudaSuccess)
       share(threads_for(n * sizeof(D)), n, [&](int, size_t lo, size_t hi) { convert(tmp + lo, dst + lo, hi - lo); });
-    std::free(tmp);
+    munmap(tmp, n * sizeof(D));
     return e;
   }
 
