@@ -61,7 +61,7 @@ class HostPipe {
   // an ensemble's `arrays` of up to `bytes` device bytes: they come in any order, and
   // slots that grow with them are paid for each time (setting 64 members: 50 ms so, 36
   // with one set of slots).  A few are all read out once before the slots are pinned
-  // (8 members 2.6 ms so, 21 with the pinning), many repay it in their first round (64
+  // (8 members 2.6 ms so, 21 with the pinning), many repay it in their first read-out (64
   // members 50 ms, 70 to 86 without).
   void expect(size_t bytes, int arrays) {
     expect_ = bytes;
@@ -179,7 +179,7 @@ class HostPipe {
   // the same rate (128^3 FP32 from FP64 1.0 to 2.3 ms either way).  Arrays out are
   // much faster through pinned ones, most of all into fresh pages (FP64, one copy /
   // pinned slots: 64x16x24 78 / 42 us, 64^3 360 / 223, 128^3 2200 / 1450, 256x256x128
-  // 14.8 / 2.7 ms), so the second array out pins (a small ensemble's second round): the
+  // 14.8 / 2.7 ms), so the second array out pins (a small ensemble's second read-out): the
   // first goes as one copy, into a temporary where it needs conversion, as handles are
   // often read out once.  Arrays of more than 32 MiB repay the pinning at once.
   cudaError_t ensure(size_t bytes, bool pin) {
